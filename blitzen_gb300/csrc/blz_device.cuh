@@ -19,6 +19,12 @@ namespace blz {
 #define BLZ_FS(a, b) __fsub_rn((a), (b))
 #define BLZ_FD(a, b) __fdiv_rn((a), (b))
 
+// A plain load, ordered after pdl_wait() (see there) and cached in L1.
+template <typename T>
+__device__ __forceinline__ T ldp(const T* p) {
+    return *p;
+}
+
 // ------------------------------------------------------------------ scalar conventions
 
 // D3D float -> uint: NaN and x <= 0 give 0, x >= 2^32 gives UINT32_MAX, else truncation.
@@ -179,10 +185,10 @@ __device__ __forceinline__ uint32_t mip_dim(uint32_t base, uint32_t level) {
 }
 
 // A pyramid texel load. COH: the pyramid was written during this launch (the one-call frame
-// kernel builds it), so the load goes to L2 (coherent), not through the read-only path.
+// kernel builds it), so the load goes to L2 (coherent), not through L1.
 template <bool COH>
 __device__ __forceinline__ float pyr_ld(const float* a) {
-    return COH ? __ldcg(a) : __ldg(a);
+    return COH ? __ldcg(a) : *a;
 }
 
 template <bool COH = false>
@@ -326,13 +332,14 @@ __device__ __forceinline__ unsigned long long load_state(const unsigned long lon
 }
 
 
-// One MeshTransform {pos.xyz, scale, quat.xyzw} in a single 256-bit read-only load (the table
-// is 32-byte aligned, checked on upload).
+// One MeshTransform {pos.xyz, scale, quat.xyzw} in a single 256-bit load (the table is 32-byte
+// aligned, checked on upload).
 __device__ __forceinline__ void ldg_transform(const BlzMeshTransform* t, float4& posScale, float4& q) {
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+    asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=f"(posScale.x), "=f"(posScale.y), "=f"(posScale.z), "=f"(posScale.w), "=f"(q.x), "=f"(q.y), "=f"(q.z),
           "=f"(q.w)
-        : "l"(t));
+        : "l"(t)
+        : "memory");
 }
 
 // Transform `tid` of the scene, from the bound dynamic rows when tid < dynCount (device or pinned
@@ -343,13 +350,16 @@ __device__ __forceinline__ void load_transform(const SceneTables& sc, uint32_t t
     ldg_transform(base + tid, posScale, q);
 }
 
-// Programmatic dependent launch. A kernel launched with programmatic stream serialization may be
-// scheduled while the kernel before it on the stream is still finishing; pdl_wait() holds it,
-// before it touches any memory, until that kernel has completed and its writes are visible (a
-// kernel launched without the attribute passes straight through). pdl_launch_next() lets the
-// next kernel on the stream be scheduled now, to wait in its own pdl_wait().
+// Programmatic dependent launch. A kernel launched with programmatic stream serialization
+// (launch_pdl) is scheduled as soon as every block of the kernel before it has ended, before that
+// kernel's end has gone through the front end; pdl_wait() holds it until that kernel has completed
+// and its writes are visible (a kernel launched without the attribute passes straight through).
+// Every thread of such a kernel calls pdl_wait() first, before it touches any memory, so a kernel
+// that has completed implies that all before it on the stream have. What a kernel before it may have
+// written (any table, list, depth buffer, count) is read after that with plain loads, never with the
+// read-only (.nc) ones, which promise the memory constant from the kernel's start and which the
+// compiler may move above the wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ void st_release_gpu(unsigned int* p, unsigned int v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");

@@ -41,7 +41,7 @@ constexpr uint32_t kClPrefixLoads = 4;   // emit launch: group and tile counts e
 __device__ __forceinline__ bool cluster_visible(const ClusterParams& p, const ViewConsts& v, const float4 posScale,
                                                 const float4 quat, uint32_t cid) {
     const float4* cp = reinterpret_cast<const float4*>(p.sc.clusters + cid);
-    const float4 sph = __ldg(cp);
+    const float4 sph = ldp(cp);
     const Vec3 w = model_to_world(Vec3{sph.x, sph.y, sph.z}, posScale, quat);
     const Vec3 c = view_transform(v.rows, w);
     const float r = BLZ_FM(sph.w, posScale.w);
@@ -51,7 +51,7 @@ __device__ __forceinline__ bool cluster_visible(const ClusterParams& p, const Vi
         if (project_sphere(c, r, v.zNear, v.proj0, v.proj5, aabb)) vis = vis && occlusion(aabb, p.pyr, v, c, r);
     }
     if (vis) {
-        const uint32_t cone = __ldg(reinterpret_cast<const uint32_t*>(cp + 1));  // int8 axis xyz, cutoff
+        const uint32_t cone = ldp(reinterpret_cast<const uint32_t*>(cp + 1));  // int8 axis xyz, cutoff
         const int ax = static_cast<int8_t>(cone & 0xFFu), ay = static_cast<int8_t>((cone >> 8) & 0xFFu);
         const int az = static_cast<int8_t>((cone >> 16) & 0xFFu), ac = static_cast<int8_t>(cone >> 24);
         const Vec3 axm{BLZ_FD(static_cast<float>(ax), 127.0f), BLZ_FD(static_cast<float>(ay), 127.0f),
@@ -90,6 +90,7 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t w, uint32_t n) {
 // items of up to kClItem clusters {object, first cluster, first slot in the tile, clusters}.
 template <bool TASKS>
 __global__ void __launch_bounds__(kClThreads) cluster_object_kernel(const ClusterParams p, const BlzCameraViewData view) {
+    pdl_wait();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t tile = blockIdx.x * kClWarps + warp;
     if (tile >= p.tiles) return;
@@ -99,15 +100,15 @@ __global__ void __launch_bounds__(kClThreads) cluster_object_kernel(const Cluste
     unsigned int flags = 0u;
     float4 posScale = make_float4(0.f, 0.f, 0.f, 1.f), quat = make_float4(0.f, 0.f, 0.f, 1.f);
     if (i < p.count) {
-        const uint2 ro = __ldg(reinterpret_cast<const uint2*>(p.objects) + i);
+        const uint2 ro = ldp(reinterpret_cast<const uint2*>(p.objects) + i);
         bool ok = ro.x < p.sc.transformCount && ro.y < p.sc.surfaceCount;
         uint4 sm = make_uint4(0u, 0u, 0u, 0u);
         float4 sph = make_float4(0.f, 0.f, 0.f, 0.f);
         if (ok) {
             load_transform(p.sc, ro.x, posScale, quat);
             const float4* sp = reinterpret_cast<const float4*>(p.sc.surfaces + ro.y);
-            sph = __ldg(sp);
-            sm = __ldg(reinterpret_cast<const uint4*>(sp + 1));
+            sph = ldp(sp);
+            sm = ldp(reinterpret_cast<const uint4*>(sp + 1));
             ok = sm.y < p.sc.lodCount && sm.z <= p.sc.lodCount - sm.y;
         }
         if (!ok) {
@@ -119,8 +120,8 @@ __global__ void __launch_bounds__(kClThreads) cluster_object_kernel(const Cluste
                 const float threshold = lod_threshold(c, r, posScale.w, v.lodTarget);
                 uint32_t idx = 0;
                 for (uint32_t k = 1; k < sm.z; ++k)
-                    if (__ldg(&p.sc.lods[sm.y + k].error) < threshold) idx = k;
-                const uint4 lod = __ldg(reinterpret_cast<const uint4*>(p.sc.lods + sm.y + idx));
+                    if (ldp(&p.sc.lods[sm.y + k].error) < threshold) idx = k;
+                const uint4 lod = ldp(reinterpret_cast<const uint4*>(p.sc.lods + sm.y + idx));
                 // lod.z = clusterOffset, lod.w = clusterCount
                 if (lod.z > p.sc.clusterCount || lod.w > p.sc.clusterCount - lod.z || lod.w > p.bitWords) {
                     // (a range longer than the longest the scene had at upload does not fit the
@@ -195,6 +196,7 @@ __device__ __forceinline__ void or_bits(uint32_t* bits, uint32_t s0, uint32_t ba
 // the order of the items), and towards the frame's totals.
 template <bool TASKS>
 __global__ void __launch_bounds__(kClThreads) cluster_test_kernel(const ClusterParams p, const BlzCameraViewData view) {
+    pdl_wait();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t nItems = min(__ldcg(p.itemCount), p.itemCapacity);
     const ViewConsts v = load_view(view);
@@ -243,6 +245,7 @@ __global__ void __launch_bounds__(kClThreads) cluster_test_kernel(const ClusterP
 // the lanes 32 at a time.
 template <bool TASKS>
 __global__ void __launch_bounds__(kClThreads) cluster_emit_kernel(const ClusterParams p) {
+    pdl_wait();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t tile = blockIdx.x * kClWarps + warp;
     if (tile >= p.tiles) return;
@@ -379,7 +382,7 @@ __global__ void __launch_bounds__(kClThreads) cluster_emit_kernel(const ClusterP
                 }
             } else if (k < roundTotal && q < p.capacity) {
                 // InitialClusterCull.comp.glsl:48-54: {objectId, triangleCount * 3, 1, dataOffset, 0, 0}
-                const uint4 meta = __ldg(reinterpret_cast<const uint4*>(p.sc.clusters + cid) + 1);
+                const uint4 meta = ldp(reinterpret_cast<const uint4*>(p.sc.clusters + cid) + 1);
                 uint32_t* rec = reinterpret_cast<uint32_t*>(p.cmds + static_cast<size_t>(q) * p.stride);
                 rec[0] = tile * kClObjects + lo;
                 rec[1] = ((meta.z >> 8) & 0xFFu) * 3u;
@@ -400,18 +403,16 @@ uint32_t cluster_tile_groups(uint32_t tiles) { return (tiles + kClSuper - 1) / k
 
 template <bool TASKS>
 static cudaError_t launch_cluster(const ClusterParams& p, const BlzCameraViewData& view, cudaStream_t s) {
-    cluster_object_kernel<TASKS><<<(p.tiles + kClWarps - 1) / kClWarps, kClThreads, 0, s>>>(p, view);
-    cudaError_t e = cudaGetLastError();
+    const uint32_t tileBlocks = (p.tiles + kClWarps - 1) / kClWarps;
+    cudaError_t e = launch_pdl(cluster_object_kernel<TASKS>, tileBlocks, kClThreads, 0, s, p, view);
     if (e != cudaSuccess) return e;
     // the test launch: every resident warp at once, or one warp per item when there are fewer
     const uint64_t maxItems = cluster_max_items(p.tiles, p.bitWords);
     uint64_t blocks = static_cast<uint64_t>(p.testBlocksPerSm > 0 ? p.testBlocksPerSm : 1) * (p.smCount > 0 ? p.smCount : 1);
     blocks = std::min<uint64_t>(blocks, (maxItems + kClWarps - 1) / kClWarps);
-    cluster_test_kernel<TASKS><<<static_cast<uint32_t>(blocks ? blocks : 1), kClThreads, 0, s>>>(p, view);
-    e = cudaGetLastError();
+    e = launch_pdl(cluster_test_kernel<TASKS>, static_cast<uint32_t>(blocks ? blocks : 1), kClThreads, 0, s, p, view);
     if (e != cudaSuccess) return e;
-    cluster_emit_kernel<TASKS><<<(p.tiles + kClWarps - 1) / kClWarps, kClThreads, 0, s>>>(p);
-    return cudaGetLastError();
+    return launch_pdl(cluster_emit_kernel<TASKS>, tileBlocks, kClThreads, 0, s, p);
 }
 
 cudaError_t cluster_test_blocks_per_sm(bool tasks, int* out) {

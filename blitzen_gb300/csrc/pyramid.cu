@@ -17,7 +17,6 @@ __global__ void __launch_bounds__(kPyrThreads) pyramid_kernel(const __grid_const
     __shared__ float sA[kPyrSmemA];
     __shared__ float sB[kPyrSmemB];
     pdl_wait();
-    pdl_launch_next();
     pyramid_tile<MODE, kPyrThreads>(p, blockIdx.x * kPyrTile, blockIdx.y * kPyrTile, sA, sB);
     // the levels above 5 span several tiles: the last block to finish builds them
     if (p.mipCount > kPyrInTileLevels + 1) pyramid_tile_finish<MODE, kPyrThreads>(p, gridDim.x * gridDim.y, p.done, nullptr, sA, sB);

@@ -161,8 +161,8 @@ __device__ __forceinline__ void pyramid_tile(const PyramidBuildParams& p, uint32
                 const uint32_t gx = X0 + 2u * (pr % (kPyrTile / 2)), gy = Y0 + pr / (kPyrTile / 2);
                 const bool in = gx < W0 && gy < H0;
                 const float4* row = reinterpret_cast<const float4*>(p.depth + static_cast<size_t>(2u * gy) * dw + 2u * gx);
-                q[j][0] = in ? __ldg(row) : make_float4(0.f, 0.f, 0.f, 0.f);
-                q[j][1] = in ? __ldg(row + dw / 4u) : make_float4(0.f, 0.f, 0.f, 0.f);
+                q[j][0] = in ? ldp(row) : make_float4(0.f, 0.f, 0.f, 0.f);
+                q[j][1] = in ? ldp(row + dw / 4u) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
 #pragma unroll
             for (uint32_t j = 0; j < PER / 2; ++j) {
@@ -186,10 +186,10 @@ __device__ __forceinline__ void pyramid_tile(const PyramidBuildParams& p, uint32
                 const bool in = gx < W0 && gy < H0;
                 const uint64_t x0 = 2ull * gx, y0 = 2ull * gy;
                 const uint32_t dw = p.depthWidth, dh = p.depthHeight;
-                q[j][0] = (in && x0 < dw && y0 < dh) ? __ldg(p.depth + y0 * dw + x0) : 0.0f;
-                q[j][1] = (in && x0 + 1 < dw && y0 < dh) ? __ldg(p.depth + y0 * dw + x0 + 1) : 0.0f;
-                q[j][2] = (in && x0 < dw && y0 + 1 < dh) ? __ldg(p.depth + (y0 + 1) * dw + x0) : 0.0f;
-                q[j][3] = (in && x0 + 1 < dw && y0 + 1 < dh) ? __ldg(p.depth + (y0 + 1) * dw + x0 + 1) : 0.0f;
+                q[j][0] = (in && x0 < dw && y0 < dh) ? ldp(p.depth + y0 * dw + x0) : 0.0f;
+                q[j][1] = (in && x0 + 1 < dw && y0 < dh) ? ldp(p.depth + y0 * dw + x0 + 1) : 0.0f;
+                q[j][2] = (in && x0 < dw && y0 + 1 < dh) ? ldp(p.depth + (y0 + 1) * dw + x0) : 0.0f;
+                q[j][3] = (in && x0 + 1 < dw && y0 + 1 < dh) ? ldp(p.depth + (y0 + 1) * dw + x0 + 1) : 0.0f;
             }
 #pragma unroll
             for (uint32_t j = 0; j < PER; ++j) v[j] = fmin_nan(q[j][0], fmin_nan(q[j][1], fmin_nan(q[j][2], q[j][3])));

@@ -10,6 +10,7 @@ namespace blz {
 // (src/Renderer/BlitzenVulkan/vulkanDraw.cpp:46-60,816-820).
 __global__ void transforms_scatter_kernel(BlzMeshTransform* table, uint32_t tableCount, const uint32_t* ids,
                                           const BlzMeshTransform* in, uint32_t n, unsigned int* status) {
+    pdl_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t id = ids[i];
@@ -29,6 +30,7 @@ __global__ void transforms_scatter_kernel(BlzMeshTransform* table, uint32_t tabl
 __global__ void transforms_rotate_kernel(const BlzMeshTransform* table, uint32_t tableCount, const BlzMeshTransform* dynRows,
                                          uint32_t dynCount, const uint32_t* ids, const float* axes, float s, float c,
                                          uint32_t n, BlzMeshTransform* dst, unsigned int* status) {
+    pdl_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t id = ids[i];
@@ -53,8 +55,7 @@ __global__ void transforms_rotate_kernel(const BlzMeshTransform* table, uint32_t
 cudaError_t launch_transforms_scatter(BlzMeshTransform* table, uint32_t tableCount, const uint32_t* ids,
                                       const BlzMeshTransform* in, uint32_t n, unsigned int* status, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    transforms_scatter_kernel<<<(n + 255) / 256, 256, 0, s>>>(table, tableCount, ids, in, n, status);
-    return cudaGetLastError();
+    return launch_pdl(transforms_scatter_kernel, (n + 255) / 256, 256, 0, s, table, tableCount, ids, in, n, status);
 }
 
 cudaError_t launch_transforms_rotate(const BlzMeshTransform* table, uint32_t tableCount, const BlzMeshTransform* dynRows,
@@ -63,9 +64,8 @@ cudaError_t launch_transforms_rotate(const BlzMeshTransform* table, uint32_t tab
     if (n == 0) return cudaSuccess;
     const float h = angle * 0.5f;
     const float sn = sinf(h), cs = cosf(h);  // host libm, the same values the host oracle uses
-    transforms_rotate_kernel<<<(n + 255) / 256, 256, 0, s>>>(table, tableCount, dynRows, dynCount, ids, axes, sn, cs, n,
-                                                               dst, status);
-    return cudaGetLastError();
+    return launch_pdl(transforms_rotate_kernel, (n + 255) / 256, 256, 0, s, table, tableCount, dynRows, dynCount, ids, axes, sn,
+                      cs, n, dst, status);
 }
 
 // ------------------------------------------------------------------ occluder raster
@@ -101,6 +101,7 @@ __device__ __forceinline__ BoxRect box_rect(const ViewConsts& v, const float* bx
 }
 
 __global__ void depth_clear_kernel(float4* depth, size_t n4, float* tail, uint32_t ntail) {
+    pdl_wait();
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n4; i += static_cast<size_t>(gridDim.x) * blockDim.x)
         depth[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (blockIdx.x == 0 && threadIdx.x < ntail) tail[threadIdx.x] = 0.0f;
@@ -112,6 +113,7 @@ __global__ void depth_clear_kernel(float4* depth, size_t n4, float* tail, uint32
 __global__ void depth_raster_kernel(const BlzCameraViewData view, const float* boxes, uint32_t boxCount, float* depth,
                                     uint32_t width, uint32_t height) {
     __shared__ BoxRect s_r;
+    pdl_wait();
     const ViewConsts v = load_view(view);
     for (uint32_t b = blockIdx.x; b < boxCount; b += gridDim.x) {
         if (threadIdx.x == 0) s_r = box_rect(v, boxes + 6 * static_cast<size_t>(b), width, height);
@@ -139,15 +141,17 @@ cudaError_t launch_depth_raster(const BlzCameraViewData& view, const float* boxe
         cudaError_t e = cudaMemsetAsync(depth, 0, n * sizeof(float), s);
         if (e != cudaSuccess) return e;
     } else {
-        depth_clear_kernel<<<1024, 256, 0, s>>>(reinterpret_cast<float4*>(depth), n4, depth + n4 * 4, ntail);
+        cudaError_t e = launch_pdl(depth_clear_kernel, 1024, 256, 0, s, reinterpret_cast<float4*>(depth), n4, depth + n4 * 4, ntail);
+        if (e != cudaSuccess) return e;
         if (launches) *launches += 1;
     }
     if (boxCount > 0) {
         const uint32_t grid = boxCount < 4096 ? boxCount : 4096;
-        depth_raster_kernel<<<grid, 256, 0, s>>>(view, boxes, boxCount, depth, width, height);
+        cudaError_t e = launch_pdl(depth_raster_kernel, grid, 256, 0, s, view, boxes, boxCount, depth, width, height);
+        if (e != cudaSuccess) return e;
         if (launches) *launches += 1;
     }
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 }  // namespace blz
