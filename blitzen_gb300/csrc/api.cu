@@ -531,9 +531,11 @@ static int pyramid_build_params(blz_ctx* c, const BlzPyramid* p, const float* de
     bp.mode = p->mode;
     for (uint32_t i = 0; i < BLZ_PYRAMID_MAX_MIPS; ++i) bp.mipOffset[i] = p->mipOffset[i];
     bp.done = &c->scratch->pyrDone;
-    bp.vec4 = (p->mode == BLZ_HIZ_D3D12 && p->depthWidth % 4 == 0 && p->depthHeight >= 2 &&
-               p->width == p->depthWidth / 2 && p->height <= p->depthHeight / 2 && p->mipOffset[0] == 0 &&
-               reinterpret_cast<uintptr_t>(depth) % 16 == 0 && reinterpret_cast<uintptr_t>(p->data) % 8 == 0) ? 1u : 0u;
+    // wide loads need every texel's 2x2 Loads inside the depth buffer, and rows that start aligned
+    const bool inside = p->mode == BLZ_HIZ_D3D12 && p->width <= p->depthWidth / 2 && p->height <= p->depthHeight / 2;
+    const uintptr_t at = reinterpret_cast<uintptr_t>(depth);
+    bp.vec = !inside ? 1u : (p->depthWidth % 4 == 0 && p->width % 2 == 0 && at % 16 == 0) ? 4u : (p->depthWidth % 2 == 0 && at % 8 == 0) ? 2u : 1u;
+    bp.pairs = (p->width % 2 == 0 && p->mipOffset[0] % 2 == 0 && reinterpret_cast<uintptr_t>(p->data) % 8 == 0) ? 1u : 0u;
     bp.spinLimit = c->waitLimit ? c->waitLimit : kSpinLimitDefault;
     return BLZ_OK;
 }

@@ -64,11 +64,8 @@ __device__ __forceinline__ float fmax_nan(float a, float b) {
     return (b > a) ? b : a;
 }
 
-__device__ __forceinline__ float fmin_nan(float a, float b) {
-    if (isnan(a)) return b;
-    if (isnan(b)) return a;
-    return (b < a) ? b : a;
-}
+// (b where a is a NaN; a where only b is; a on a tie)
+__device__ __forceinline__ float fmin_nan(float a, float b) { return (isnan(a) || b < a) ? b : a; }
 
 // ------------------------------------------------------------------ sphere math
 

@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) cull_frame_kernel(con
         __syncthreads();
         const uint32_t t = s_tile;
         if (t >= tiles) break;
-        pyramid_tile<HIZ, THREADS>(bp, (t % tilesX) * kPyrTile, (t / tilesX) * kPyrTile, sA, sB);
+        pyramid_tile<HIZ, THREADS>(bp, (t % tilesX) * kPyrTile, (t / tilesX) * kPyrTile, sA);
         pyramid_tile_finish<HIZ, THREADS>(bp, tiles, &scr->frameTilesDone, &scr->frameReady, sA, sB);
         __syncthreads();  // s_tile and the tile buffers are free again
     }

@@ -199,7 +199,8 @@ struct PyramidBuildParams {
     uint32_t width, height, mipCount, mode;
     uint32_t mipOffset[BLZ_PYRAMID_MAX_MIPS];
     unsigned int* done;  // the context's finished-tile counter (zero between builds)
-    uint32_t vec4;       // D3D12: depth rows read 16 bytes at a time (width % 4 == 0, height >= 2, aligned buffers)
+    uint32_t vec;        // D3D12: depth floats read at a time, 4 or 2 (the row length and the buffer's alignment allow it), or 1
+    uint32_t pairs;      // mip 0 written two texels at a time (its width is even and its storage 8-byte aligned)
     uint32_t spinLimit;  // one-call frame kernel: polls of the pyramid-ready flag before a warp gives up
 };
 
