@@ -223,7 +223,8 @@ int blz_ctx_create(int device, blz_ctx** out) {
     cudaDeviceGetAttribute(&c->smCount, cudaDevAttrMultiProcessorCount, device);
     c->stateCapacity = kDefaultStateCapacity;
     const size_t bytes = kScratchHeaderBytes + c->stateCapacity * sizeof(unsigned long long);
-    e = cudaMalloc(&c->scratchMem, bytes);
+    const size_t rectOffset = (bytes + 255) & ~size_t(255);
+    e = cudaMalloc(&c->scratchMem, rectOffset + kRasterScratchBytes);
     if (e != cudaSuccess) { delete c; return e == cudaErrorMemoryAllocation ? fail(BLZ_ERR_OUT_OF_MEMORY, "scratch allocation failed") : cuda_fail(e, "cudaMalloc scratch"); }
     e = cudaMemset(c->scratchMem, 0, bytes);
     if (e == cudaSuccess) {
@@ -242,6 +243,7 @@ int blz_ctx_create(int device, blz_ctx** out) {
         return rc;
     }
     c->scratch = static_cast<Scratch*>(c->scratchMem);
+    c->rectScratch = static_cast<char*>(c->scratchMem) + rectOffset;
     *out = c;
     return BLZ_OK;
 }
@@ -560,7 +562,8 @@ int blz_depth_raster_boxes(blz_ctx* c, const BlzCameraViewData* view, const floa
     if (boxCount && !boxes) return fail(BLZ_ERR_INVALID_ARGUMENT, "boxes is NULL");
     if (width == 0 || height == 0 || (uint64_t)width * height >= (1ull << 31)) return fail(BLZ_ERR_INVALID_ARGUMENT, "bad depth extent");
     uint32_t launches = 0;
-    cudaError_t e = launch_depth_raster(*view, boxes, boxCount, depth, width, height, reinterpret_cast<cudaStream_t>(stream), &launches);
+    cudaError_t e = launch_depth_raster(*view, boxes, boxCount, depth, width, height, c->rectScratch,
+                                        reinterpret_cast<cudaStream_t>(stream), &launches);
     if (e != cudaSuccess) return cuda_fail(e, "depth raster launch");
     c->launches += launches;
     return BLZ_OK;

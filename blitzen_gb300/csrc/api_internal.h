@@ -35,6 +35,7 @@ struct blz_ctx {
     void* scratchMem = nullptr;        // Scratch header + tile states
     blz::Scratch* scratch = nullptr;
     size_t stateCapacity = 0;
+    void* rectScratch = nullptr;       // box raster: kRasterScratchBytes at the end of scratchMem
     unsigned int* workCounter = nullptr;  // batch decide launches: next chunk (zero between launches)
     void* pinned = nullptr;            // pinned host staging
     cudaEvent_t pinnedDone = nullptr;  // last copy out of `pinned` has completed

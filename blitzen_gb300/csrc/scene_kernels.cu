@@ -75,29 +75,41 @@ struct BoxRect {
     float depth;
 };
 
-__device__ __forceinline__ BoxRect box_rect(const ViewConsts& v, const float* bx, uint32_t width, uint32_t height) {
-    BoxRect r{0, 0, 0, 0, 0.0f};
-    const float fw = static_cast<float>(width), fh = static_cast<float>(height);
-    float minx = INFINITY, maxx = -INFINITY, miny = INFINITY, maxy = -INFINITY, zmax = -INFINITY;
-    for (int k = 0; k < 8; ++k) {
-        const Vec3 p{bx[(k & 1) ? 3 : 0], bx[(k & 2) ? 4 : 1], bx[(k & 4) ? 5 : 2]};
-        const Vec3 q = view_transform(v.rows, p);
-        if (!(q.z > v.zNear)) return r;  // boxes reaching the near plane are skipped
-        const float sx = BLZ_FM(BLZ_FA(BLZ_FM(BLZ_FD(BLZ_FM(q.x, v.proj0), q.z), 0.5f), 0.5f), fw);
-        const float sy = BLZ_FM(BLZ_FS(0.5f, BLZ_FM(BLZ_FD(BLZ_FM(q.y, v.proj5), q.z), 0.5f)), fh);
-        minx = fmin_nan(minx, sx);
-        maxx = fmax_nan(maxx, sx);
-        miny = fmin_nan(miny, sy);
-        maxy = fmax_nan(maxy, sy);
-        zmax = fmax_nan(zmax, q.z);
-    }
+// Screen position of a box corner (view space).
+__device__ __forceinline__ void box_corner(const ViewConsts& v, Vec3 q, uint32_t width, uint32_t height, float& sx, float& sy) {
+    sx = BLZ_FM(BLZ_FA(BLZ_FM(BLZ_FD(BLZ_FM(q.x, v.proj0), q.z), 0.5f), 0.5f), static_cast<float>(width));
+    sy = BLZ_FM(BLZ_FS(0.5f, BLZ_FM(BLZ_FD(BLZ_FM(q.y, v.proj5), q.z), 0.5f)), static_cast<float>(height));
+}
+
+// The pixel rectangle of the corners' extent, clipped to the screen, and its depth.
+__device__ __forceinline__ BoxRect box_extent(const ViewConsts& v, float minx, float miny, float maxx, float maxy, float zmax,
+                                              uint32_t width, uint32_t height) {
+    BoxRect r;
     r.depth = BLZ_FD(v.zNear, zmax);
+    const float fw = static_cast<float>(width), fh = static_cast<float>(height);
     const float fx0 = floorf(minx), fy0 = floorf(miny), fx1 = ceilf(maxx), fy1 = ceilf(maxy);
     r.x0 = fx0 < 0.0f ? 0 : (fx0 > fw ? static_cast<int>(width) : static_cast<int>(fx0));
     r.y0 = fy0 < 0.0f ? 0 : (fy0 > fh ? static_cast<int>(height) : static_cast<int>(fy0));
     r.x1 = fx1 < 0.0f ? 0 : (fx1 > fw ? static_cast<int>(width) : static_cast<int>(fx1));
     r.y1 = fy1 < 0.0f ? 0 : (fy1 > fh ? static_cast<int>(height) : static_cast<int>(fy1));
     return r;
+}
+
+__device__ __forceinline__ BoxRect box_rect(const ViewConsts& v, const float* bx, uint32_t width, uint32_t height) {
+    float minx = INFINITY, maxx = -INFINITY, miny = INFINITY, maxy = -INFINITY, zmax = -INFINITY;
+    for (int k = 0; k < 8; ++k) {
+        const Vec3 p{bx[(k & 1) ? 3 : 0], bx[(k & 2) ? 4 : 1], bx[(k & 4) ? 5 : 2]};
+        const Vec3 q = view_transform(v.rows, p);
+        if (!(q.z > v.zNear)) return BoxRect{0, 0, 0, 0, 0.0f};  // boxes reaching the near plane are skipped
+        float sx, sy;
+        box_corner(v, q, width, height, sx, sy);
+        minx = fmin_nan(minx, sx);
+        maxx = fmax_nan(maxx, sx);
+        miny = fmin_nan(miny, sy);
+        maxy = fmax_nan(maxy, sy);
+        zmax = fmax_nan(zmax, q.z);
+    }
+    return box_extent(v, minx, miny, maxx, maxy, zmax, width, height);
 }
 
 __global__ void depth_clear_kernel(float4* depth, size_t n4, float* tail, uint32_t ntail) {
@@ -132,8 +144,146 @@ __global__ void depth_raster_kernel(const BlzCameraViewData view, const float* b
     }
 }
 
+// The screen tiles of the other form: one block per kTileW x kTileH pixels, a warp per 32x16 of them, 16
+// pixels a thread (four neighbours in each of four rows). The block keeps the boxes whose rectangle meets its tile (every box
+// tested once per tile, up to kTileHits at a time), takes the largest depth over each pixel in registers and
+// writes the pixel once, the cleared ones included: the image is written once and never read, where the
+// block per box clears it and then sends one atomic a covered pixel.
+// 2000 boxes of the stress scene's sizes at 3840x2160: 13 us a raster (2.8 rectangles, 12.0 tiles, in a
+// stream) against 32; 8192 boxes of 1 to 4 units there, the tile form's worst: 25 against 28, and
+// since a tile tests every box, that is where the dispatch's line lies.
+constexpr uint32_t kTileW = 64, kTileH = 64;  // (128 x 64: 16.1 us a tile launch against 12.0: a warp meets more boxes it has no pixel of)
+constexpr uint32_t kTileThreads = kTileW / 4u * kTileH / 4u;
+constexpr uint32_t kTileHits = 1024;
+constexpr uint32_t kTileScan = 4;  // rectangles a thread loads at a time
+constexpr uint32_t kTilePart = kTileHits / kTileThreads;  // of which this many join the list before it is used
+constexpr uint32_t kRasterTileExtent = 1u << 16;  // a side whose tiles fit a launch grid
+static_assert(kTileHits % kTileThreads == 0 && kTileScan % kTilePart == 0, "whole parts");
+
+// box_rect by eight lanes, one per corner (the same corners compared in the same order).
+__global__ void __launch_bounds__(128) box_rects_kernel(const BlzCameraViewData view, const float* boxes, uint32_t boxCount,
+                                                        uint32_t width, uint32_t height, int4* rects, int* depths) {
+    pdl_wait();
+    const uint32_t at = blockIdx.x * 16u + threadIdx.x / 8u, k = threadIdx.x % 8u;
+    const uint32_t b = min(at, boxCount - 1u);
+    const ViewConsts v = load_view(view);
+    const float* bx = boxes + 6 * static_cast<size_t>(b);
+    const Vec3 q = view_transform(v.rows, Vec3{bx[(k & 1u) ? 3 : 0], bx[(k & 2u) ? 4 : 1], bx[(k & 4u) ? 5 : 2]});
+    float minx, miny, maxx, maxy, zmax = q.z;
+    box_corner(v, q, width, height, minx, miny);
+    maxx = minx;
+    maxy = miny;
+    const unsigned front = __ballot_sync(0xFFFFFFFFu, q.z > v.zNear);
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) {  // the lower corner's value first, as in box_rect
+        const bool low = (k & static_cast<uint32_t>(d)) == 0u;
+        auto pair = [&](float x, auto op) {
+            const float o = __shfl_xor_sync(0xFFFFFFFFu, x, d);
+            return low ? op(x, o) : op(o, x);
+        };
+        minx = pair(minx, [](float l, float h) { return fmin_nan(l, h); });
+        maxx = pair(maxx, [](float l, float h) { return fmax_nan(l, h); });
+        miny = pair(miny, [](float l, float h) { return fmin_nan(l, h); });
+        maxy = pair(maxy, [](float l, float h) { return fmax_nan(l, h); });
+        zmax = pair(zmax, [](float l, float h) { return fmax_nan(l, h); });
+    }
+    if (k != 0u || at >= boxCount) return;
+    const uint32_t lane = threadIdx.x & 31u;
+    BoxRect r{0, 0, 0, 0, 0.0f};
+    if (((front >> lane) & 0xFFu) == 0xFFu)  // boxes reaching the near plane are skipped
+        r = box_extent(v, fmin_nan(INFINITY, minx), fmin_nan(INFINITY, miny), fmax_nan(-INFINITY, maxx), fmax_nan(-INFINITY, maxy),
+                       fmax_nan(-INFINITY, zmax), width, height);
+    const bool drawn = r.x1 > r.x0 && r.y1 > r.y0 && r.depth > 0.0f;
+    rects[b] = drawn ? make_int4(r.x0, r.y0, r.x1, r.y1) : make_int4(0, 0, 0, 0);
+    depths[b] = __float_as_int(r.depth);
+}
+
+__global__ void __launch_bounds__(kTileThreads) depth_tiles_kernel(const int4* rects, const int* depths, uint32_t boxCount,
+                                                                   float* depth, uint32_t width, uint32_t height, uint32_t vec4) {
+    __shared__ int4 s_rect[kTileHits];
+    __shared__ int s_depth[kTileHits];
+    __shared__ uint32_t s_hits;
+    pdl_wait();
+    const int X0 = static_cast<int>(blockIdx.x * kTileW), Y0 = static_cast<int>(blockIdx.y * kTileH);
+    const int lane = static_cast<int>(threadIdx.x & 31u), warp = static_cast<int>(threadIdx.x >> 5);
+    const int wx = X0 + warp % static_cast<int>(kTileW / 32u) * 32, wy = Y0 + warp / static_cast<int>(kTileW / 32u) * 16;
+    const int x = wx + lane % 8 * 4, y = wy + lane / 8;  // rows y, y + 4, y + 8, y + 12
+    int v[4][4];  // depths are positive: the largest float has the largest bits
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[j][i] = 0;
+    for (uint32_t first = 0; first < boxCount; first += kTileThreads * kTileScan) {
+        int4 r[kTileScan];
+#pragma unroll
+        for (uint32_t k = 0; k < kTileScan; ++k) {
+            const uint32_t b = first + k * kTileThreads + threadIdx.x;
+            r[k] = b < boxCount ? rects[b] : make_int4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (uint32_t part = 0; part < kTileScan; part += kTilePart) {
+            if (first + part * kTileThreads >= boxCount) break;  // (the whole block)
+            __syncthreads();                                     // the list before this one is done with
+            if (threadIdx.x == 0) s_hits = 0u;
+            __syncthreads();
+#pragma unroll
+            for (uint32_t k = part; k < part + kTilePart; ++k) {
+                if (r[k].x < X0 + static_cast<int>(kTileW) && r[k].z > X0 && r[k].y < Y0 + static_cast<int>(kTileH) && r[k].w > Y0) {
+                    const uint32_t at = atomicAdd(&s_hits, 1u);
+                    s_rect[at] = r[k];
+                    s_depth[at] = depths[first + k * kTileThreads + threadIdx.x];
+                }
+            }
+            __syncthreads();
+            const uint32_t n = s_hits;
+            for (uint32_t h = 0; h < n; ++h) {
+                const int4 q = s_rect[h];
+                if (q.x >= wx + 32 || q.z <= wx || q.y >= wy + 16 || q.w <= wy) continue;  // (the whole warp)
+                const int d = s_depth[h];
+                int c[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) c[i] = x + i >= q.x && x + i < q.z ? d : 0;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int row = y + 4 * j;
+                    if (row >= q.y && row < q.w) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) v[j][i] = max(v[j][i], c[i]);
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int row = y + 4 * j;
+        if (row >= static_cast<int>(height)) continue;
+        float* out = depth + static_cast<size_t>(row) * width + x;
+        if (vec4) {  // the width is a multiple of 4: the four are in the row or none is
+            if (x < static_cast<int>(width)) *reinterpret_cast<int4*>(out) = make_int4(v[j][0], v[j][1], v[j][2], v[j][3]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (x + i < static_cast<int>(width)) out[i] = __int_as_float(v[j][i]);
+        }
+    }
+}
+
 cudaError_t launch_depth_raster(const BlzCameraViewData& view, const float* boxes, uint32_t boxCount, float* depth,
-                                uint32_t width, uint32_t height, cudaStream_t s, uint32_t* launches) {
+                                uint32_t width, uint32_t height, void* rectScratch, cudaStream_t s, uint32_t* launches) {
+    if (boxCount > 0 && boxCount <= kRasterTileBoxes && width <= kRasterTileExtent && height <= kRasterTileExtent) {
+        int4* rects = static_cast<int4*>(rectScratch);
+        int* depths = reinterpret_cast<int*>(rects + kRasterTileBoxes);
+        cudaError_t e = launch_pdl(box_rects_kernel, (boxCount + 15) / 16, 128, 0, s, view, boxes, boxCount, width, height, rects, depths);
+        if (e != cudaSuccess) return e;
+        const dim3 grid((width + kTileW - 1) / kTileW, (height + kTileH - 1) / kTileH);
+        const uint32_t vec4 = width % 4u == 0u && reinterpret_cast<uintptr_t>(depth) % 16 == 0 ? 1u : 0u;
+        e = launch_pdl(depth_tiles_kernel, grid, kTileThreads, 0, s, static_cast<const int4*>(rects), static_cast<const int*>(depths),
+                       boxCount, depth, width, height, vec4);
+        if (e != cudaSuccess) return e;
+        if (launches) *launches += 2;
+        return cudaSuccess;
+    }
     const size_t n = static_cast<size_t>(width) * height;
     const size_t n4 = (reinterpret_cast<uintptr_t>(depth) % 16 == 0) ? n / 4 : 0;
     const uint32_t ntail = static_cast<uint32_t>(n - n4 * 4);
