@@ -190,6 +190,25 @@ int cluster_test_occupancy(blz_ctx* c, bool tasks, ClusterParams& p) {
     return BLZ_OK;
 }
 
+// Scratch of the instanced cull of scenes of many LODs, a block of its own: recorded calls never use it
+// (see blz_cull_instanced), so it can grow whatever has been recorded.
+static int ensure_many_lods_scratch(blz_ctx* c, size_t bytes) {
+    if (bytes <= c->manyLodsBytes) return BLZ_OK;
+    if (c->manyLodsMem) {
+        cudaDeviceSynchronize();
+        cudaFree(c->manyLodsMem);
+        c->manyLodsMem = nullptr;
+        c->manyLodsBytes = 0;
+    }
+    const size_t want = bytes + bytes / 4;
+    if (cudaMalloc(&c->manyLodsMem, want) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return fail(BLZ_ERR_OUT_OF_MEMORY, "instanced scratch of %zu bytes", want);
+    }
+    c->manyLodsBytes = want;
+    return BLZ_OK;
+}
+
 void bind_chunk_scratch(blz_ctx* c, PipeParams& p) {
     char* m = static_cast<char*>(c->chunkMem);
     p.staged = reinterpret_cast<uint2*>(m);
@@ -242,6 +261,10 @@ int blz_ctx_create(int device, blz_ctx** out) {
         blz_ctx_destroy(c);
         return rc;
     }
+    if (ensure_many_lods_scratch(c, kFirstManyLodsBytes) != BLZ_OK) {
+        blz_ctx_destroy(c);
+        return fail(BLZ_ERR_OUT_OF_MEMORY, "scratch allocation failed");
+    }
     c->scratch = static_cast<Scratch*>(c->scratchMem);
     c->rectScratch = static_cast<char*>(c->scratchMem) + rectOffset;
     *out = c;
@@ -260,6 +283,7 @@ int blz_ctx_destroy(blz_ctx* c) {
     if (c->batchDev) cudaFree(c->batchDev);
     if (c->chunkMem) cudaFree(c->chunkMem);
     if (c->instScratch) cudaFree(c->instScratch);
+    if (c->manyLodsMem) cudaFree(c->manyLodsMem);
     if (c->clusterMem) cudaFree(c->clusterMem);
     if (c->frameMem) cudaFree(c->frameMem);
     delete c;
@@ -909,6 +933,41 @@ int blz_cull_frame(blz_ctx* c, const BlzCameraViewData* view, BlzRenderList list
     return BLZ_OK;
 }
 
+}  // extern "C"
+
+namespace blz {
+
+// Whether `s` is being recorded into a graph, by blz_capture_begin or by anyone else.
+static bool stream_capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return true;
+    }
+    return st != cudaStreamCaptureStatusNone;
+}
+
+// The group histograms and totals of scenes of up to kInstStagedMaxLods LODs.
+static int ensure_instanced_words(blz_ctx* c, size_t words) {
+    if (words <= c->instWords) return BLZ_OK;
+    if (c->capturing) return fail(BLZ_ERR_CAPACITY, "scratch must grow, which a capture cannot record: run the call once before capturing");
+    if (c->instScratch) {
+        cudaDeviceSynchronize();
+        cudaFree(c->instScratch);
+        c->instScratch = nullptr;
+        c->instWords = 0;
+    }
+    const size_t want = words + words / 4;
+    if (cudaMalloc(&c->instScratch, want * sizeof(uint32_t)) != cudaSuccess)
+        return fail(BLZ_ERR_OUT_OF_MEMORY, "instanced scratch of %zu bytes", want * sizeof(uint32_t));
+    c->instWords = want;
+    return BLZ_OK;
+}
+
+}  // namespace blz
+
+extern "C" {
+
 int blz_cull_instanced(blz_ctx* c, const BlzCameraViewData* view, BlzRenderList list, BlzLodInstanceCounter* counters,
                        uint32_t* instances, uint32_t instanceCapacity, uint32_t slotsPerLod, const BlzCullTarget* target,
                        blz_stream_t s) {
@@ -924,28 +983,33 @@ int blz_cull_instanced(blz_ctx* c, const BlzCameraViewData* view, BlzRenderList 
     const uint32_t nL = c->scene.lodCount;
     if (nL == 0) return fail(BLZ_ERR_INVALID_ARGUMENT, "the scene has no LODs");
     if (nL > kMaxInstancedLods) return fail(BLZ_ERR_INVALID_ARGUMENT, "instanced cull supports up to %u LODs, scene has %u", kMaxInstancedLods, nL);
-    if (nL <= kInstStagedMaxLods) {
-        // the FRUSTUM decide kernel stages (object, LOD) pairs; a counting sort turns them into lists
-        const uint32_t tile = single_chunk_size(kModeInstanced, c->singleThreads, c->singleOpt, count, c->smCount);
-        uint32_t chunks = (count + tile - 1) / tile;
-        if (chunks == 0) chunks = 1;
-        rc = ensure_chunk_scratch(c, chunks, tile);
+    const bool manyLods = nL > kInstStagedMaxLods;
+    if (manyLods) {
+        const uint32_t tiles = (count + instanced_tile_size() - 1) / instanced_tile_size();
+        rc = ensure_states(c, (size_t)(tiles ? tiles : 1) * nL);
         if (rc != BLZ_OK) return rc;
-        const uint32_t groups = instanced_group_count(chunks);
-        const size_t words = static_cast<size_t>(groups) * nL;  // the groups' LOD histograms
-        if (words > c->instWords) {
-            if (c->capturing) return fail(BLZ_ERR_CAPACITY, "scratch must grow, which a capture cannot record: run the call once before capturing");
-            if (c->instScratch) {
-                cudaDeviceSynchronize();
-                cudaFree(c->instScratch);
-                c->instScratch = nullptr;
-                c->instWords = 0;
-            }
-            const size_t want = words + words / 4;
-            if (cudaMalloc(&c->instScratch, want * sizeof(uint32_t)) != cudaSuccess)
-                return fail(BLZ_ERR_OUT_OF_MEMORY, "instanced scratch of %zu bytes", want * sizeof(uint32_t));
-            c->instWords = want;
-        }
+    }
+    // the FRUSTUM decide kernel stages (object, LOD) pairs; a counting sort turns them into lists
+    const uint32_t tile = single_chunk_size(kModeInstanced, c->singleThreads, c->singleOpt, count, c->smCount);
+    uint32_t chunks = (count + tile - 1) / tile;
+    if (chunks == 0) chunks = 1;
+    const uint32_t groups = instanced_group_count(chunks);
+    // Scenes of many LODs also have a form that needs no scratch, one launch in which tiles wait for one
+    // another: 38 us against 15 for 250k objects and 2000 LODs, but a recorded call keeps it, since it
+    // needs no earlier call to have sized anything and stays valid whatever grows later, and so does a call
+    // whose scratch the device has no room for.
+    const size_t words = static_cast<size_t>(groups + 1u) * nL;  // the groups' histograms, then the LODs' totals
+    const size_t staged = static_cast<size_t>(chunks) * tile;
+    bool sorted = true;
+    if (!manyLods) {
+        rc = ensure_chunk_scratch(c, chunks, tile);
+        if (rc == BLZ_OK) rc = ensure_instanced_words(c, words);
+        if (rc != BLZ_OK) return rc;
+    } else {
+        sorted = !stream_capturing(reinterpret_cast<cudaStream_t>(s)) &&
+                 ensure_many_lods_scratch(c, staged * sizeof(uint2) + (chunks + words) * sizeof(uint32_t)) == BLZ_OK;
+    }
+    if (sorted) {
         PipeParams p{};
         p.sc = c->scene;
         p.single.view = *view;
@@ -956,8 +1020,12 @@ int blz_cull_instanced(blz_ctx* c, const BlzCameraViewData* view, BlzRenderList 
         p.totalTiles = chunks;
         p.chunkSize = tile;
         bind_chunk_scratch(c, p);
+        if (manyLods) {
+            p.staged = static_cast<uint2*>(c->manyLodsMem);
+            p.chunkCount = reinterpret_cast<uint32_t*>(p.staged + staged);
+        }
         p.workCounter = nullptr;
-        p.instHist = c->instScratch;
+        p.instHist = manyLods ? p.chunkCount + chunks : c->instScratch;
         p.instLods = nL;
         InstStagedParams q{};
         q.staged = p.staged;
@@ -966,7 +1034,8 @@ int blz_cull_instanced(blz_ctx* c, const BlzCameraViewData* view, BlzRenderList 
         q.chunkSize = tile;
         q.groups = groups;
         q.nL = nL;
-        q.hist = c->instScratch;
+        q.hist = p.instHist;
+        q.totals = p.instHist + static_cast<size_t>(groups) * nL;
         q.lods = c->scene.lods;
         q.counters = counters;
         q.instances = instances;
@@ -977,14 +1046,15 @@ int blz_cull_instanced(blz_ctx* c, const BlzCameraViewData* view, BlzRenderList 
         q.capacity = target->capacity;
         q.drawCount = target->drawCount;
         q.status = &c->scratch->status;
+        if (manyLods) {
+            q.ticket = &c->scratch->ticket;
+            q.ticketDone = &c->scratch->doneBlocks;
+        }
         cudaError_t e = launch_instanced_staged(p, q, c->singleThreads, c->singleOpt, c->smCount, reinterpret_cast<cudaStream_t>(s));
         if (e != cudaSuccess) return cuda_fail(e, "instanced cull launch");
-        c->launches += 2;  // decide (with the group histograms), place
+        c->launches += 4;  // the group histograms' zeroing, decide, scan, place
         return BLZ_OK;
     }
-    const uint32_t tiles = (count + instanced_tile_size() - 1) / instanced_tile_size();
-    rc = ensure_states(c, (size_t)(tiles ? tiles : 1) * nL);
-    if (rc != BLZ_OK) return rc;
     InstancedParams p{};
     p.sc = c->scene;
     p.objects = objs;

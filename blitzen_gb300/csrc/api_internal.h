@@ -14,6 +14,7 @@ namespace blz {
 
 constexpr size_t kDefaultStateCapacity = size_t(1) << 22;  // 4M tile states (32 MiB)
 constexpr size_t kPinnedBytes = size_t(8) << 20;            // pinned host staging: transform rows, batch views
+constexpr size_t kFirstManyLodsBytes = size_t(4) << 20;     // many-LOD instanced scratch of a new context
 constexpr uint32_t kMaxInstancedLods = 4096;                // shared-memory bucket histograms
 
 // An autotuner's choice for one workload size: batches keyed by (total objects, views), single-view
@@ -44,8 +45,10 @@ struct blz_ctx {
     void* chunkMem = nullptr;          // object-cull staging: records, chunk counts
     size_t chunkObjects = 0;           // staged-record capacity
     size_t chunkSlots = 0;             // chunk count capacity
-    uint32_t* instScratch = nullptr;   // instanced cull: group x LOD counts, then LOD totals
+    uint32_t* instScratch = nullptr;   // instanced cull: group x LOD counts, then LOD totals (up to kInstStagedMaxLods LODs)
     size_t instWords = 0;
+    void* manyLodsMem = nullptr;       // instanced cull above kInstStagedMaxLods LODs: staged records, chunk counts, histograms, totals
+    size_t manyLodsBytes = 0;
     void* clusterMem = nullptr;        // cluster cull: tile counts, object ranges and survivors, visibility bits
     size_t clusterBytes = 0;
     int clusterTestBlocksPerSm[2] = {0, 0};  // records, task form: resident test blocks per SM (found on first use)

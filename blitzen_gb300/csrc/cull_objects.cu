@@ -69,7 +69,10 @@ __device__ __forceinline__ uint32_t find_view_warp(const uint32_t* tileStart, ui
 // ------------------------------------------------------------------ decisions
 
 constexpr uint32_t kChunk = 512;  // objects per chunk of batched views (single views size theirs)
-constexpr uint32_t kInstGroup = 32;  // chunks per group of the instanced counting sort, one warp each
+// Chunks per group of the instanced counting sort. 16 and 8 took 46.0 and 48.7 us against 44.9 for the
+// instanced pass of 4M objects and 256 LODs, 24.5 and 31.3 against 18.6 for 250k and 2000 (more rows to
+// scan, fewer warps to place them).
+constexpr uint32_t kInstGroup = 32;
 
 // A frustum survivor waiting for the dense stage (32 bytes, two 16-byte shared-memory words).
 struct Survivor {
@@ -975,89 +978,146 @@ cudaError_t launch_object_cull(uint32_t mode, const PipeParams& p, uint32_t thre
 // frustum + LOD pass decides: every visible object and its LOD. So it runs that decide kernel
 // (kModeInstanced), whose staged (objectId, lodId) records are in object order per chunk and which
 // also counts each group's records per LOD (hist[group][lod], groups of kInstGroup chunks, zeroed
-// before the launch), and then one place launch, a block per group:
-//   offsets  each LOD's offset for the group is the sum of the LOD's counts in the groups before it
-//            (coalesced loads across LODs, the block's threads taking interleaved groups); the last
-//            group's block adds its own group's counts, which gives every LOD's total, and writes
-//            the counters and, in ascending LOD order, one command per non-empty LOD;
-//   rows     each warp counts its chunk's records per LOD, and the block scans those rows per LOD;
-//   place    each warp places its records in order (ranks inside 32-record slices from one
-//            ballot per bit of the LOD id).
+// before the launch), and then two launches:
+//   scan   every LOD's counts scanned over the groups, in place: hist[group][lod] becomes the group's
+//          offset in the LOD's list; totals[lod] the list's length;
+//   place  a block per group: each warp counts its chunks' records per LOD (a row of counts in shared
+//          memory), the block scans the rows per LOD, and each warp places its records in order (ranks
+//          inside 32-record slices from one ballot per bit of the LOD id). The last group's block writes
+//          the counters and, in ascending LOD order, one command per non-empty LOD.
+// A row of counts takes 4 bytes a LOD, so scenes of more LODs get fewer warps a block, each with more
+// of the group's chunks (inst_warps). All three launches are latency chains of a few block phases; 4M
+// objects and 256 LODs: decide 33, scan 3.1, place 9.6 us (11.4 when each place block summed the earlier
+// groups' counts itself); 250k objects and 2000 LODs: 6.2, 2.9 and 10.0 us, against 37 us for the one
+// launch whose tiles look back over one another's counts of every LOD (cull_instanced.cu).
 
 constexpr uint32_t kInstBatch = 5;  // 32-record slices whose loads are issued together (the first batch's ranks are kept)
-constexpr uint32_t kInstThreads = kInstGroup * 32;
+constexpr uint32_t kInstMaxPerWarp = 4;  // chunks of a group one warp takes at most
+constexpr uint32_t kScanLods = 32, kScanParts = 32, kScanKeep = 8;
 
-
-__global__ void __launch_bounds__(kInstThreads) inst_place_kernel(const InstStagedParams q) {
+__global__ void __launch_bounds__(kScanLods* kScanParts) inst_scan_kernel(uint32_t* hist, uint32_t* totals, uint32_t groups, uint32_t nL) {
+    __shared__ uint32_t s_part[kScanParts][kScanLods];
     pdl_wait();
-    // [kInstGroup][nL] per-warp counts, then offsets; [nL] the group's offset in each LOD's list;
-    // [nL] each LOD's instanceOffset; [nL] (the last group's block) each LOD's total; [R][nL] partial sums
-    extern __shared__ uint32_t s_rows[];
+    const uint32_t l = threadIdx.x % kScanLods, part = threadIdx.x / kScanLods, lod = blockIdx.x * kScanLods + l;
+    const uint32_t per = (groups + kScanParts - 1u) / kScanParts;
+    const uint32_t g0 = min(groups, part * per), g1 = min(groups, g0 + per);
+    const bool in = lod < nL;
+    // the part's first kScanKeep counts stay in registers, loaded together
+    uint32_t keep[kScanKeep], sum = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kScanKeep; ++k) {
+        keep[k] = in && g0 + k < g1 ? __ldcg(hist + static_cast<size_t>(g0 + k) * nL + lod) : 0u;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < kScanKeep; ++k) sum += keep[k];
+    for (uint32_t g = g0 + kScanKeep; in && g < g1; ++g) sum += __ldcg(hist + static_cast<size_t>(g) * nL + lod);
+    s_part[part][l] = sum;
+    __syncthreads();
+    if (!in) return;
+    uint32_t run = 0;
+    for (uint32_t q = 0; q < part; ++q) run += s_part[q][l];
+    if (part == kScanParts - 1u) totals[lod] = run + sum;
+#pragma unroll
+    for (uint32_t k = 0; k < kScanKeep; ++k) {
+        if (g0 + k < g1) hist[static_cast<size_t>(g0 + k) * nL + lod] = run;
+        run += keep[k];
+    }
+    for (uint32_t g = g0 + kScanKeep; g < g1; ++g) {
+        uint32_t* h = hist + static_cast<size_t>(g) * nL + lod;
+        const uint32_t c = __ldcg(h);
+        *h = run;
+        run += c;
+    }
+}
+
+// Words of a row of per-LOD counts: a multiple of 4, so that the rows are scanned four LODs at a time.
+__host__ __device__ __forceinline__ uint32_t inst_stride(uint32_t nL) { return (nL + 3u) & ~3u; }
+
+// Parts the rows are scanned in by T threads, each thread four LODs of one part (0: one, no partial sums).
+__host__ __device__ __forceinline__ uint32_t inst_parts(uint32_t nL, uint32_t T) {
+    const uint32_t r = T / (inst_stride(nL) / 4u);
+    return r >= 8u ? 8u : (r >= 4u ? 4u : (r >= 2u ? 2u : 0u));
+}
+
+constexpr uint32_t kInstSmem = 220u * 1024u;
+
+// Warps of a place block for nL LODs: what 220 KB of shared memory hold rows for, a power of two.
+static uint32_t inst_warps(uint32_t nL) {
+    const uint32_t rows = kInstSmem / 4u / inst_stride(nL);  // W + 2 rows, and the scan's parts
+    uint32_t w = kInstGroup;
+    while (w > kInstGroup / kInstMaxPerWarp && w + 2u + inst_parts(nL, w * 32u) > rows) w /= 2u;
+    return w;
+}
+
+__global__ void __launch_bounds__(kInstGroup * 32) inst_place_kernel(const InstStagedParams q) {
+    // rows of nS words: [W] per-warp counts, then offsets; the group's offset in each LOD's list; each
+    // LOD's instanceOffset; [R] partial sums
+    extern __shared__ __align__(16) uint32_t s_rows[];
     __shared__ unsigned int s_flags;
     __shared__ uint32_t s_warpSums[32];
-    const uint32_t nL = q.nL, G = q.groups, g = blockIdx.x;
+    __shared__ uint32_t s_group;
+    pdl_wait();
+    const uint32_t T = blockDim.x, W = T / 32u, per = kInstGroup / W;
+    const uint32_t nL = q.nL, nS = inst_stride(nL), G = q.groups;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    uint32_t* s_goff = s_rows + kInstGroup * nL;
-    uint32_t* s_ioff = s_goff + nL;
-    uint32_t* s_tot = s_ioff + nL;
-    uint32_t* s_part = s_tot + nL;
-    // thread t works on LOD t % nL as row t / nL of R rows (nL <= kInstStagedMaxLods <= kInstThreads)
-    const uint32_t R = kInstThreads / nL;
-    const uint32_t tb = threadIdx.x % nL, tr = threadIdx.x / nL;
-    const uint32_t chunk = g * kInstGroup + warp;
-    const uint32_t n = chunk < q.totalTiles ? __ldcg(q.chunkCount + chunk) : 0u;
-    const uint2* st = q.staged + static_cast<size_t>(chunk) * q.chunkSize;
+    uint32_t* s_goff = s_rows + W * nS;
+    uint32_t* s_ioff = s_goff + nS;
+    uint32_t* s_part = s_ioff + nS;
+    if (threadIdx.x == 0) {
+        s_flags = 0u;
+        s_group = q.ticket ? atomicAdd(q.ticket, 1u) : blockIdx.x;
+    }
+    for (uint32_t j = threadIdx.x; j < W * nS / 4u; j += T) reinterpret_cast<uint4*>(s_rows)[j] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    const uint32_t g = s_group;
+    const bool held = g < G;  // else a place past the grid: the tickets were left advanced
+    unsigned int flags = held ? 0u : BLZ_FLAG_TIMEOUT;
+    // the warp's records: those of its `per` chunks, one after another
+    const uint32_t c0 = g * kInstGroup + warp * per;
+    uint32_t first[kInstMaxPerWarp], n = 0;  // record index each chunk starts at
+#pragma unroll
+    for (uint32_t k = 0; k < kInstMaxPerWarp; ++k) {
+        first[k] = n;
+        if (held && k < per && c0 + k < q.totalTiles) n += __ldcg(q.chunkCount + c0 + k);
+    }
+    auto record = [&](uint32_t j) -> uint2 {
+        uint32_t k = 0, from = 0;
+#pragma unroll
+        for (uint32_t t = 1; t < kInstMaxPerWarp; ++t)
+            if (t < per && j >= first[t]) k = t, from = first[t];
+        return __ldcg(q.staged + static_cast<size_t>(c0 + k) * q.chunkSize + (j - from));
+    };
     auto load_batch = [&](uint32_t j0, uint2 (&r)[kInstBatch]) {
 #pragma unroll
         for (uint32_t k = 0; k < kInstBatch; ++k) {
             const uint32_t j = j0 + k * 32u + lane;
-            r[k] = j < n ? __ldcg(st + j) : make_uint2(0u, 0xFFFFFFFFu);
+            r[k] = j < n ? record(j) : make_uint2(0u, 0xFFFFFFFFu);
         }
     };
-    uint2 first[kInstBatch];  // the chunk's first kInstBatch * 32 records, loaded once for both walks
-    load_batch(0, first);
-    // LOD threadIdx.x's instanceOffset (nL <= kInstThreads), stored to shared memory once phase 1
-    // is done, so no barrier waits for the load
-    const uint32_t ioff = threadIdx.x < nL ? ldp(&q.counters[threadIdx.x].instanceOffset) : 0u;
+    uint2 head[kInstBatch];  // the warp's first kInstBatch * 32 records, loaded once for both walks
+    load_batch(0, head);
     const uint32_t idBits = nL > 1u ? 32u - static_cast<uint32_t>(__clz(static_cast<int>(nL - 1u))) : 0u;
-    for (uint32_t b = threadIdx.x; b < nL; b += kInstThreads) {
-        s_goff[b] = 0u;
-        s_tot[b] = 0u;
+    for (uint32_t b = threadIdx.x; b < nL; b += T) {
+        s_goff[b] = held ? __ldcg(q.hist + static_cast<size_t>(g) * nL + b) : 0u;
+        s_ioff[b] = __ldcg(&q.counters[b].instanceOffset);
     }
-    for (uint32_t j = threadIdx.x; j < kInstGroup * nL; j += kInstThreads) s_rows[j] = 0u;
-    if (threadIdx.x == 0) s_flags = 0u;
-    __syncthreads();
-    // 0. the group's offset in each LOD's list: the LOD's counts of the groups before this one,
-    //    row tr taking every R-th group (coalesced across LODs)
-    if (tr < R) {
-        const uint32_t g1 = g;
-        uint32_t sum = 0, gg = tr;
-        for (; gg + 7u * R < g1; gg += 8u * R) {  // eight loads in flight at a time
-            uint32_t x[8];
-#pragma unroll
-            for (uint32_t k = 0; k < 8u; ++k) x[k] = __ldcg(q.hist + static_cast<size_t>(gg + k * R) * nL + tb);
-#pragma unroll
-            for (uint32_t k = 0; k < 8u; ++k) sum += x[k];
-        }
-        for (; gg < g1; gg += R) sum += __ldcg(q.hist + static_cast<size_t>(gg) * nL + tb);
-        if (sum) atomicAdd(&s_goff[tb], sum);
-    }
-    uint32_t* row = s_rows + warp * nL;
+    uint32_t* row = s_rows + warp * nS;
     const uint32_t lt = lanemask_lt();
-    // 1. this chunk's records per LOD (only this warp touches its row); each of the first batch's
-    //    records also keeps its rank among the chunk's records of its LOD (the count before its
+    // 1. the warp's records per LOD (only this warp touches its row); each of the first batch's
+    //    records also keeps its rank among the warp's records of its LOD (the count before its
     //    32-record slice, from the slice's lowest lane of that LOD, plus the lanes below it)
     uint32_t rank[kInstBatch];
     for (uint32_t j0 = 0; j0 < n; j0 += 32u * kInstBatch) {
         uint2 r[kInstBatch];
         if (j0 == 0) {
 #pragma unroll
-            for (uint32_t k = 0; k < kInstBatch; ++k) r[k] = first[k];
+            for (uint32_t k = 0; k < kInstBatch; ++k) r[k] = head[k];
         } else {
             load_batch(j0, r);
         }
 #pragma unroll
         for (uint32_t k = 0; k < kInstBatch; ++k) {
+            if (j0 + k * 32u >= n) break;  // (the whole warp)
             const uint32_t b = r[k].y;
             const unsigned peers = same_lod_lanes(b, idBits, b != 0xFFFFFFFFu);
             uint32_t before = 0;
@@ -1072,55 +1132,70 @@ __global__ void __launch_bounds__(kInstThreads) inst_place_kernel(const InstStag
             __syncwarp();
         }
     }
-    if (threadIdx.x < nL) s_ioff[threadIdx.x] = ioff;
     __syncthreads();
-    // 2. per LOD, exclusive offsets of the warps' chunks inside the group: row tr of threads sums
-    //    its kInstGroup / R consecutive warps' counts, then scans them after the sums of the rows
-    //    before it
-    const uint32_t per = (kInstGroup + R - 1u) / R;
-    const uint32_t w0 = min(kInstGroup, tr * per), w1 = min(kInstGroup, w0 + per);
-    if (tr < R) {
-        uint32_t part = 0;
-        for (uint32_t w = w0; w < w1; ++w) part += s_rows[w * nL + tb];
-        s_part[tr * nL + tb] = part;
-    }
-    __syncthreads();
-    if (tr < R) {
-        uint32_t run = 0;
-        for (uint32_t r = 0; r < tr; ++r) run += s_part[r * nL + tb];
-        for (uint32_t w = w0; w < w1; ++w) {
-            const uint32_t c = s_rows[w * nL + tb];
-            s_rows[w * nL + tb] = run;
-            run += c;
+    // 2. per LOD, exclusive offsets of the warps' records: the group's offset and the counts of the warps
+    //    before, four LODs a thread; R parts of the rows at a time when there are threads for them, each
+    //    starting from the sums of the parts before it
+    {
+        const uint32_t Q = nS / 4u, R = inst_parts(nL, T);
+        auto add = [](uint4& x, const uint4 y) { x.x += y.x, x.y += y.y, x.z += y.z, x.w += y.w; };
+        auto at = [&](uint32_t* rows, uint32_t i, uint32_t b) -> uint4& { return reinterpret_cast<uint4*>(rows + i * nS)[b]; };
+        auto scan = [&](uint4 run, uint32_t w0, uint32_t w1, uint32_t b) {
+            for (uint32_t w = w0; w < w1; w += 4u) {
+                uint4 c[4];
+#pragma unroll
+                for (uint32_t k = 0; k < 4u; ++k) c[k] = w + k < w1 ? at(s_rows, w + k, b) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+                for (uint32_t k = 0; k < 4u; ++k) {
+                    if (w + k < w1) at(s_rows, w + k, b) = run;
+                    add(run, c[k]);
+                }
+            }
+        };
+        if (R == 0u) {
+            for (uint32_t b = threadIdx.x; b < Q; b += T) scan(at(s_goff, 0, b), 0u, W, b);
+        } else {
+            const uint32_t b = threadIdx.x % Q, part = threadIdx.x / Q, span = W / R;  // W and R are powers of two, R <= W
+            if (part < R) {
+                uint4 sum = make_uint4(0u, 0u, 0u, 0u);
+                for (uint32_t w = part * span; w < part * span + span; ++w) add(sum, at(s_rows, w, b));
+                at(s_part, part, b) = sum;
+            }
+            __syncthreads();
+            if (part < R) {
+                uint4 run = at(s_goff, 0, b);
+                for (uint32_t k = 0; k < part; ++k) add(run, at(s_part, k, b));
+                scan(run, part * span, part * span + span, b);
+            }
         }
     }
     __syncthreads();
-    // 3. place the records in object order: a chunk the first batch holds whole places each record
-    //    at its LOD's group offset + the warp's offset + its rank; a longer one ranks its records
-    //    again, slice by slice
+    // 3. place the records in object order: a warp whose records the first batch holds places each at its
+    //    LOD's offset for the warp + its rank; a longer one ranks its records again, slice by slice
     const uint32_t slots = q.slotsPerLod ? q.slotsPerLod : 0xFFFFFFFFu;
-    unsigned int flags = 0u;
+    auto put = [&](uint32_t obj, uint32_t b, uint32_t pos) {
+        const uint64_t at = static_cast<uint64_t>(s_ioff[b]) + pos;
+        if (pos < slots && at < q.instanceCapacity) q.instances[at] = obj;
+        else flags |= BLZ_FLAG_INSTANCE_OVERFLOW;
+    };
     if (n <= 32u * kInstBatch) {
 #pragma unroll
         for (uint32_t k = 0; k < kInstBatch; ++k) {
-            const uint32_t b = first[k].y;
-            if (b == 0xFFFFFFFFu) continue;
-            const uint32_t pos = s_goff[b] + row[b] + rank[k];
-            const uint64_t at = static_cast<uint64_t>(s_ioff[b]) + pos;
-            if (pos < slots && at < q.instanceCapacity) q.instances[at] = first[k].x;
-            else flags |= BLZ_FLAG_INSTANCE_OVERFLOW;
+            const uint32_t b = head[k].y;
+            if (b != 0xFFFFFFFFu) put(head[k].x, b, row[b] + rank[k]);
         }
     }
     for (uint32_t j0 = 0; n > 32u * kInstBatch && j0 < n; j0 += 32u * kInstBatch) {
         uint2 r[kInstBatch];
         if (j0 == 0) {
 #pragma unroll
-            for (uint32_t k = 0; k < kInstBatch; ++k) r[k] = first[k];
+            for (uint32_t k = 0; k < kInstBatch; ++k) r[k] = head[k];
         } else {
             load_batch(j0, r);
         }
 #pragma unroll
         for (uint32_t k = 0; k < kInstBatch; ++k) {
+            if (j0 + k * 32u >= n) break;  // (the whole warp)
             const uint32_t b = r[k].y;
             const unsigned peers = same_lod_lanes(b, idBits, b != 0xFFFFFFFFu);
             uint32_t before = 0;
@@ -1128,25 +1203,18 @@ __global__ void __launch_bounds__(kInstThreads) inst_place_kernel(const InstStag
             __syncwarp();
             if (b != 0xFFFFFFFFu) {
                 if ((peers & lt) == 0u) row[b] = before + __popc(peers);
-                const uint32_t pos = s_goff[b] + before + __popc(peers & lt);
-                const uint64_t at = static_cast<uint64_t>(s_ioff[b]) + pos;
-                if (pos < slots && at < q.instanceCapacity) q.instances[at] = r[k].x;
-                else flags |= BLZ_FLAG_INSTANCE_OVERFLOW;
+                put(r[k].x, b, before + __popc(peers & lt));
             }
             __syncwarp();
         }
     }
-    // 4. the last group's block: every LOD's total is its group offset plus its own group's count;
-    //    then the counters and, in ascending LOD order, one command per non-empty LOD
+    // 4. the last group's block: the counters and, in ascending LOD order, one command per non-empty LOD
     //    (drawInstCmd.cs.hlsl:9-38)
     if (g == G - 1u) {
-        for (uint32_t l = threadIdx.x; l < nL; l += kInstThreads)
-            s_tot[l] = s_goff[l] + __ldcg(q.hist + static_cast<size_t>(g) * nL + l);
-        __syncthreads();
-        const uint32_t perT = (nL + kInstThreads - 1u) / kInstThreads;
+        const uint32_t perT = (nL + T - 1u) / T;
         const uint32_t b0 = min(nL, threadIdx.x * perT), b1 = min(nL, b0 + perT);
         uint32_t mine = 0;
-        for (uint32_t l = b0; l < b1; ++l) mine += s_tot[l] ? 1u : 0u;
+        for (uint32_t l = b0; l < b1; ++l) mine += __ldcg(q.totals + l) ? 1u : 0u;
         uint32_t incl = mine;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -1156,13 +1224,13 @@ __global__ void __launch_bounds__(kInstThreads) inst_place_kernel(const InstStag
         if (lane == 31) s_warpSums[warp] = incl;
         __syncthreads();
         uint32_t warpOff = 0, all = 0;
-        for (uint32_t w = 0; w < 32u; ++w) {
+        for (uint32_t w = 0; w < W; ++w) {
             if (w < warp) warpOff += s_warpSums[w];
             all += s_warpSums[w];
         }
         uint32_t out = warpOff + incl - mine;
         for (uint32_t l = b0; l < b1; ++l) {
-            const uint32_t total = s_tot[l];
+            const uint32_t total = __ldcg(q.totals + l);
             q.counters[l].instanceCount = total;
             const uint32_t offset = s_ioff[l];
             if (total > slots || static_cast<uint64_t>(offset) + min(total, slots) > q.instanceCapacity)
@@ -1185,7 +1253,17 @@ __global__ void __launch_bounds__(kInstThreads) inst_place_kernel(const InstStag
     }
     if (flags) atomicOr(&s_flags, flags);
     __syncthreads();
-    if (threadIdx.x == 0 && s_flags) atomicOr(q.status, s_flags);
+    if (threadIdx.x == 0) {
+        if (s_flags) atomicOr(q.status, s_flags);
+        // the block that ends last rewinds the tickets
+        if (q.ticket) {
+            __threadfence();
+            if (atomicAdd(q.ticketDone, 1u) == G - 1u) {
+                *q.ticket = 0u;
+                *q.ticketDone = 0u;
+            }
+        }
+    }
 }
 
 __global__ void __launch_bounds__(1024) zero_words_kernel(uint32_t* words, uint32_t n) {
@@ -1208,12 +1286,15 @@ cudaError_t launch_instanced_staged(const PipeParams& p, const InstStagedParams&
     else if (threads == 512 && opt == 1) e = launch_decide_t<kModeInstanced, true, 512, 1>(p, 0, smCount, s);
     else e = launch_decide_t<kModeInstanced, true, kObjThreads, kObjOpt>(p, 0, smCount, s);
     if (e != cudaSuccess) return e;
-    const size_t rowBytes = sizeof(uint32_t) * ((kInstGroup + 3) * q.nL + (kInstThreads / q.nL) * q.nL);
+    e = launch_pdl(inst_scan_kernel, (q.nL + kScanLods - 1) / kScanLods, kScanLods * kScanParts, 0, s, p.instHist, q.totals, q.groups, q.nL);
+    if (e != cudaSuccess) return e;
+    const uint32_t warps = inst_warps(q.nL), threads32 = warps * 32u;
+    const size_t rowBytes = sizeof(uint32_t) * (warps + 2u + inst_parts(q.nL, threads32)) * inst_stride(q.nL);
     if (rowBytes > 48 * 1024) {
         e = cudaFuncSetAttribute(inst_place_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(rowBytes));
         if (e != cudaSuccess) return e;
     }
-    return launch_pdl(inst_place_kernel, q.groups, kInstThreads, rowBytes, s, q);
+    return launch_pdl(inst_place_kernel, q.groups, threads32, rowBytes, s, q);
 }
 
 bool batch_shape_supported(uint32_t threads, uint32_t opt) {

@@ -145,7 +145,8 @@ struct InstStagedParams {
     const uint32_t* chunkCount; // [totalTiles]
     uint32_t totalTiles, chunkSize;
     uint32_t groups, nL;        // chunk groups of the counting sort, LOD count
-    const uint32_t* hist;       // [groups][nL] record counts per group and LOD (the decide kernel's)
+    const uint32_t* hist;       // [groups][nL] each group's offset in each LOD's list (the scan launch's)
+    uint32_t* totals;           // [nL] each LOD's record count (the scan launch's)
     const BlzLodData* lods;
     BlzLodInstanceCounter* counters;
     uint32_t* instances;
@@ -154,6 +155,8 @@ struct InstStagedParams {
     uint32_t stride, capacity;
     uint32_t* drawCount;
     unsigned int* status;
+    unsigned int* ticket;       // groups are taken from this counter (zero between launches), or NULL: block g takes group g
+    unsigned int* ticketDone;   // blocks that have ended (zero between launches)
 };
 
 struct ClusterParams {
@@ -249,7 +252,9 @@ bool batch_shape_supported(uint32_t threads, uint32_t opt);
 cudaError_t launch_batch_cull(const PipeParams& p, uint32_t threads, uint32_t opt, uint32_t blocksPerSm, int smCount,
                               cudaStream_t s, int mode);
 uint32_t instanced_tile_size();
-constexpr uint32_t kInstStagedMaxLods = 1024;  // the staged instanced path keeps [36 to 39][LODs] words in shared memory
+// Above this many LODs the instanced cull's place launch takes its groups by ticket, and a recorded call
+// runs as one launch without scratch (launch_instanced_cull).
+constexpr uint32_t kInstStagedMaxLods = 1024;
 uint32_t instanced_group_count(uint32_t chunks);
 cudaError_t launch_instanced_staged(const PipeParams& p, const InstStagedParams& q, uint32_t threads, uint32_t opt,
                                     int smCount, cudaStream_t s);
