@@ -23,9 +23,12 @@ from .abi import BlzError, CameraViewData, CullTarget, Pyramid, RenderList, Scen
 from .scenes import Scene
 
 
-def _stream_ptr(stream: torch.cuda.Stream | None) -> C.c_void_p:
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+def _stream_ptr(stream: torch.cuda.Stream | None) -> int:
+    """The cudaStream_t of `stream`, or of torch's current stream on the current device. Read through the
+    raw getter: building a torch.cuda.Stream object for it takes 2.9 us of a call's 10, this 0.2."""
+    if stream is not None:
+        return stream.cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _dev_u32(n: int, device) -> torch.Tensor:
