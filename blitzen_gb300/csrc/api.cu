@@ -103,7 +103,8 @@ int ensure_chunk_scratch(blz_ctx* c, size_t chunks, size_t chunkSize) {
         c->chunkMem = nullptr;
         c->chunkObjects = c->chunkSlots = 0;
     }
-    const size_t bytes = wantObj * sizeof(uint2) + wantSlots * sizeof(uint32_t) + 256;
+    // staged records; per chunk its count, its place (uint2) and its turn (the last two: batches)
+    const size_t bytes = wantObj * sizeof(uint2) + wantSlots * 4 * sizeof(uint32_t) + 256;
     if (cudaMalloc(&c->chunkMem, bytes) != cudaSuccess) return fail(BLZ_ERR_OUT_OF_MEMORY, "object-cull scratch of %zu bytes", bytes);
     c->chunkObjects = wantObj;
     c->chunkSlots = wantSlots;
@@ -212,7 +213,8 @@ static int ensure_many_lods_scratch(blz_ctx* c, size_t bytes) {
 void bind_chunk_scratch(blz_ctx* c, PipeParams& p) {
     char* m = static_cast<char*>(c->chunkMem);
     p.staged = reinterpret_cast<uint2*>(m);
-    p.chunkCount = reinterpret_cast<uint32_t*>(m + c->chunkObjects * sizeof(uint2));
+    p.chunkBase = p.staged + c->chunkObjects;
+    p.chunkCount = reinterpret_cast<uint32_t*>(p.chunkBase + c->chunkSlots);
     p.workCounter = c->workCounter;
     p.scratch = c->scratch;
 }

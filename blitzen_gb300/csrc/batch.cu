@@ -143,6 +143,19 @@ static int uniform_mode(const BlzBatchView* views, uint32_t n) {
     return n ? static_cast<int>(views[0].mode) : -1;
 }
 
+// Whether the chunks are decided in the order of batch_order_kernel: several views, enough chunks for it to
+// matter, and a transform table that would be read from memory again for each view.
+static bool wants_order(const PipeParams& p) {
+    return p.viewCount > 1 && p.viewCount <= kBatchOrderViews && p.totalTiles >= kBatchOrderChunks &&
+           p.sc.transformCount * sizeof(BlzMeshTransform) >= kBatchOrderBytes;
+}
+
+static uint32_t largest_view(const std::vector<uint32_t>& tileStart) {
+    uint32_t most = 0;
+    for (size_t i = 1; i < tileStart.size(); ++i) most = std::max(most, tileStart[i] - tileStart[i - 1]);
+    return most;
+}
+
 static int run_batch_shape(blz_ctx* c, const BlzBatchView* views, uint32_t n, cudaStream_t st, const BlzLaunchShape& sh) {
     const uint32_t tile = batch_chunk(sh);
     std::vector<BatchViewDev> d;
@@ -157,10 +170,17 @@ static int run_batch_shape(blz_ctx* c, const BlzBatchView* views, uint32_t n, cu
     rc = upload_views(c, d, ts, c->batchDev, st, tile, p);
     if (rc != BLZ_OK) return rc;
     bind_chunk_scratch(c, p);
-    cudaError_t e = launch_batch_cull(p, sh.threadsPerBlock, sh.objectsPerThread, sh.blocksPerSm, c->smCount, st,
-                                      uniform_mode(views, n));
+    cudaError_t e = cudaSuccess;
+    if (wants_order(p)) {
+        uint32_t* order = p.chunkCount + c->chunkSlots;
+        e = launch_batch_order(p, largest_view(ts), order, st);
+        p.order = order;
+        c->launches++;
+    }
+    if (e == cudaSuccess)
+        e = launch_batch_cull(p, sh.threadsPerBlock, sh.objectsPerThread, sh.blocksPerSm, c->smCount, st, uniform_mode(views, n));
     if (e != cudaSuccess) return cuda_fail(e, "batch launch");
-    c->launches += 2;  // decide + scatter
+    c->launches += 3;  // decide, scan, scatter
     return BLZ_OK;
 }
 
@@ -367,15 +387,22 @@ int blz_batch_graph_create(blz_ctx* c, const BlzBatchView* views, uint32_t n, bl
     if (rc == BLZ_OK && cudaStreamSynchronize(st) != cudaSuccess) rc = fail(BLZ_ERR_CUDA, "batch graph upload failed");
     if (rc == BLZ_OK) {
         const size_t chunks = ts[n], objects = chunks * tile;
-        const size_t bytes = objects * sizeof(uint2) + chunks * sizeof(uint32_t) + 256;
+        const size_t bytes = objects * sizeof(uint2) + chunks * 4 * sizeof(uint32_t) + 256;
         if (cudaMalloc(&g->chunkMem, bytes) != cudaSuccess || cudaMemset(g->chunkMem, 0, bytes) != cudaSuccess) {
             rc = fail(BLZ_ERR_OUT_OF_MEMORY, "batch graph scratch allocation failed");
         } else {
             char* m = static_cast<char*>(g->chunkMem);
             p.staged = reinterpret_cast<uint2*>(m);
-            p.chunkCount = reinterpret_cast<uint32_t*>(m + objects * sizeof(uint2));
-            p.workCounter = reinterpret_cast<unsigned int*>(p.chunkCount + chunks);  // zeroed above
+            p.chunkBase = p.staged + objects;
+            p.chunkCount = reinterpret_cast<uint32_t*>(p.chunkBase + chunks);
+            uint32_t* order = p.chunkCount + chunks;
+            p.workCounter = reinterpret_cast<unsigned int*>(order + chunks);  // zeroed above
             p.scratch = c->scratch;
+            if (wants_order(p)) {  // it depends on the lists' sizes alone, which the graph keeps
+                p.order = order;
+                if (launch_batch_order(p, largest_view(ts), order, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
+                    rc = fail(BLZ_ERR_CUDA, "batch graph order failed");
+            }
         }
     }
     cudaStream_t cap = nullptr;
@@ -411,7 +438,7 @@ int blz_batch_graph_launch(blz_batch_graph* g, blz_stream_t stream) {
     if (!g || !g->exec) return fail(BLZ_ERR_INVALID_ARGUMENT, "graph is NULL");
     cudaError_t e = cudaGraphLaunch(g->exec, reinterpret_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(e, "graph launch");
-    g->ctx->launches += 2;
+    g->ctx->launches += 3;
     return BLZ_OK;
 }
 

@@ -150,6 +150,66 @@ __device__ __forceinline__ bool frustum_check(Vec3 c, float r, const ViewConsts&
     return vis;
 }
 
+// ------------------------------------------------------------------ reject test
+//
+// Most objects of a frame lie outside the frustum, and the exact test needs the rotated sphere centre
+// in the shaders' operation order: 75 instructions. This one proves most of them outside from the
+// object's position alone. With m the model sphere's centre, S the scale, R the quaternion's matrix,
+// the exact test sees c = V (pos + S R m) + w, and c differs from pc = V pos + w by at most
+// |row_i| |S| K |m| in component i, where K = max(1, 2 |q|^2 - 1) bounds |R m| / |m|: the quaternion
+// formula leaves the part of m along q as it is and scales the rest by sqrt(1 + 4 |q.xyz|^2 (|q|^2 - 1)).
+// So a plane's exact value cannot exceed its value at pc by more than a |S| K |m|, a = the largest over
+// the planes of the sum of |plane coefficient| |row|. Rounding: the exact chain and this one together
+// stay within 16 u (u = 2^-24) of the sums of magnitudes they add, at most s M (|x|+|y|+|z|) + s W for
+// the position terms (M, W the largest view coefficient and translation, s the largest sum of plane
+// coefficients), 64 u being allowed for them, and within 110 u of |S| K |m| for the rotation, where a
+// carries a factor of 1 + 2^-9. An object is dropped when some plane's value at pc is below
+// -T, T = r + 64 u |r| + a |S| K |m| + b (|x|+|y|+|z|) + d: then the exact comparison fails too. A NaN
+// or an overflow makes T or the plane's value NaN or infinite, and the object is not dropped, or the
+// exact test has the same NaN in that plane and fails. Dropping is the only thing decided here.
+constexpr float kRejectUlps = 3.814697265625e-6f;  // 64 u
+
+struct RejectBounds {
+    float a, b, d;
+};
+
+__device__ __forceinline__ RejectBounds reject_bounds(const ViewConsts& v) {
+    const ViewRows& m = v.rows;
+    auto norm = [](float4 r) { return sqrtf(r.x * r.x + r.y * r.y + r.z * r.z); };
+    auto top = [](float4 r) { return fmaxf(fabsf(r.x), fmaxf(fabsf(r.y), fabsf(r.z))); };
+    const float n0 = norm(m.r0), n1 = norm(m.r1), n2 = norm(m.r2);
+    const float fl = fabsf(v.frustumLeft), fr = fabsf(v.frustumRight), fb = fabsf(v.frustumBottom), ft = fabsf(v.frustumTop);
+    const float s = fmaxf(1.0f, fmaxf(fl + fr, fb + ft));
+    const float big = fmaxf(top(m.r0), fmaxf(top(m.r1), top(m.r2)));
+    const float far = fmaxf(fabsf(m.r0.w), fmaxf(fabsf(m.r1.w), fabsf(m.r2.w)));
+    RejectBounds rj;
+    rj.a = 1.001953125f * fmaxf(n2, fmaxf(fl * n2 + fr * n0, fb * n2 + ft * n1)) + 1e-18f;
+    rj.b = kRejectUlps * s * big;
+    rj.d = kRejectUlps * s * far + 1e-30f;
+    return rj;
+}
+
+// What the reject test needs of a surface: its radius and a bound of |m| (the 1-norm), or a NaN, with
+// which no object is ever dropped, for a surface whose LOD range is bad (the exact stage reports it).
+__device__ __forceinline__ float2 surface_bound(float4 sphere, bool lodOk) {
+    return make_float2(sphere.w, lodOk ? fabsf(sphere.x) + fabsf(sphere.y) + fabsf(sphere.z) : __int_as_float(0x7fc00000));
+}
+
+__device__ __forceinline__ bool surely_outside(float4 ps, float4 q, float2 surface, const ViewConsts& v, const RejectBounds& rj) {
+    const ViewRows& m = v.rows;
+    const float x = __fmaf_rn(m.r0.x, ps.x, __fmaf_rn(m.r0.y, ps.y, __fmaf_rn(m.r0.z, ps.z, m.r0.w)));
+    const float y = __fmaf_rn(m.r1.x, ps.x, __fmaf_rn(m.r1.y, ps.y, __fmaf_rn(m.r1.z, ps.z, m.r1.w)));
+    const float z = __fmaf_rn(m.r2.x, ps.x, __fmaf_rn(m.r2.y, ps.y, __fmaf_rn(m.r2.z, ps.z, m.r2.w)));
+    const float n = __fmaf_rn(q.x, q.x, __fmaf_rn(q.y, q.y, __fmaf_rn(q.z, q.z, q.w * q.w)));
+    const float k = fmaxf(1.0f, __fmaf_rn(2.0f, n, -1.0f));
+    const float r = surface.x * ps.w;
+    const float off = fabsf(ps.w) * surface.y * k;
+    const float t = __fmaf_rn(rj.a, off, __fmaf_rn(rj.b, fabsf(ps.x) + fabsf(ps.y) + fabsf(ps.z), __fmaf_rn(kRejectUlps, fabsf(r), r) + rj.d));
+    const float side = __fmaf_rn(z, v.frustumLeft, -(fabsf(x) * v.frustumRight));
+    const float updown = __fmaf_rn(z, v.frustumBottom, -(fabsf(y) * v.frustumTop));
+    return fminf(fminf(side, updown), fminf(z - v.zNear, v.zFar - z)) < -t;
+}
+
 // hlslMath.hlsl:30-56 (ProjectSphere), CullingShaderData.glsl:8-33. aabb in UV space, y flipped.
 __device__ __forceinline__ bool project_sphere(Vec3 c, float r, float znear, float P00, float P11, float4& aabb) {
     if (c.z < BLZ_FA(r, znear)) return false;
@@ -356,7 +416,14 @@ __device__ __forceinline__ void load_transform(const SceneTables& sc, uint32_t t
 // written (any table, list, depth buffer, count) is read after that with plain loads, never with the
 // read-only (.nc) ones, which promise the memory constant from the kernel's start and which the
 // compiler may move above the wait.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#ifndef BLZ_TRIG
+#define BLZ_TRIG 0
+#endif
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory");
+#if BLZ_TRIG
+ asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#endif
+}
 
 __device__ __forceinline__ void st_release_gpu(unsigned int* p, unsigned int v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");

@@ -1,15 +1,15 @@
 // cull_objects.cu — per-object cull kernels: frustum, occlusion pass 1 / pass 2, temporal
 // occlusion, for one view or many views in one launch.
 //
-// Two kernels per launch, no block ever waiting on another:
+// Two or three kernels per launch, no block ever waiting on another:
 //   decide   a streaming grid of warps, each deciding contiguous chunks of a view's render objects
 //            (single views: one chunk per resident warp, assigned by warp index; batches: 512-object
 //            chunks of all views, taken from a work counter), staging the emitted ones compacted in
 //            object order — (objectId, lodId), 8 bytes — in the chunk's slice of a scratch buffer,
 //            with the chunk's count;
-//   scatter  one block per 32 chunks: the block finds its chunks' output offsets from the counts
-//            (no grid-wide scan), copies the staged records to their final slots as full indirect
-//            records, and the owner of each view's last chunk writes the view's draw count.
+//   scatter  finds the chunks' output offsets from the counts, copies the staged records to their final
+//            slots as full indirect records and writes the draw count (single views: one block per 32
+//            chunks; batches: a scan launch, a block per view, then one warp per chunk).
 // The scratch traffic is 16 bytes per emitted object, against 40-48 bytes read per object.
 //
 // Reference passes (paths inside the Blitzen project):
@@ -38,18 +38,8 @@ __device__ __forceinline__ const BatchViewDev& view_of(const PipeParams& p, uint
     }
 }
 
-// Chunk c belongs to the view v with tileStart[v] <= c < tileStart[v + 1].
-__device__ __forceinline__ uint32_t find_view(const uint32_t* tileStart, uint32_t nViews, uint32_t c) {
-    uint32_t lo = 0, hi = nViews;
-    while (hi - lo > 1u) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (ldp(tileStart + mid) <= c) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
-
-// The same for a chunk index c that is equal on every lane of the warp: a 32-ary search, one round
+// Chunk c belongs to the view v with tileStart[v] <= c < tileStart[v + 1]; c is equal on every lane of the
+// warp: a 32-ary search, one round
 // of loads per factor of 32 views instead of one dependent load per halving.
 __device__ __forceinline__ uint32_t find_view_warp(const uint32_t* tileStart, uint32_t nViews, uint32_t c) {
     const uint32_t lane = threadIdx.x & 31u;
@@ -74,14 +64,34 @@ constexpr uint32_t kChunk = 512;  // objects per chunk of batched views (single 
 // scan, fewer warps to place them).
 constexpr uint32_t kInstGroup = 32;
 
-// A frustum survivor waiting for the dense stage (32 bytes, two 16-byte shared-memory words).
+// Where the reject test (surely_outside) comes before the exact frustum test, and the exact test runs in the
+// dense stage, on the objects the bound cannot drop: the one-call frame and batched views. The frame of 4M
+// objects took 52.3 us without and 48.8 with it, a batch of 64 views 300 and 287. The other
+// single-view passes test every object exactly where it is loaded: most of their lists are short or, in
+// pass 1, mostly inside the frustum, and the second stage's latency cost 0.2 to 0.9 us of passes of 100k to
+// 1M objects (at 4M the instanced pass gained 0.2 us).
+__host__ __device__ constexpr bool reject_mode(int mode, bool single) { return !single || mode == 5 || mode == 6; }
+static_assert(kModeFrameFused == 5 && kModeFramePyr == 6, "reject_mode names the fused modes");
+
+// A warp's queue of objects waiting for the dense stage, in shared memory.
+constexpr uint32_t kRing = 64;  // slots: under 32 waiting plus one 32-object slice
+template <bool REJECT>
+struct Ring {
+    // object index within the view and, in bits 30-31, min(visibility word, 2); then
+    // REJECT: surface id, pos.xy | pos.z, scale, quat.xy | quat.zw; else: view-space centre | r, scale, LOD range
+    uint4 a[kRing];
+    uint4 b[kRing];
+    uint2 c[REJECT ? kRing : 1u];
+};
+constexpr uint32_t kBadObject = 0xFFFFFFFFu;  // in place of the surface id: a transform or surface id was out of range
+
+// A frustum survivor pass 1 of a kept frame hands to pass 2 (32 bytes, two 16-byte words).
 struct Survivor {
-    uint32_t obj;      // object index within the view; bit 31: visible last frame (LATE)
+    uint32_t obj;      // object index within the view (bit 31: visibility word was not 0, bit 30: it was 1)
     float cx, cy, cz;  // view-space sphere centre
     float r, scale;
     uint32_t lodOff, lodCnt;
 };
-constexpr uint32_t kRing = 64;  // per-warp survivor ring: under 32 waiting plus one 32-object slice
 
 // Both passes of a frame decided in one sweep, with the pyramid built before the launch or inside it.
 __host__ __device__ constexpr bool fused_mode(int m) { return m == kModeFrameFused || m == kModeFramePyr; }
@@ -114,115 +124,163 @@ __device__ __forceinline__ unsigned same_lod_lanes(uint32_t b, uint32_t bits, bo
     return m;
 }
 
-// Dense stage over one survivor per lane (lanes with `mine`), in object order: the sphere
-// projection and Hi-Z test (LATE/TEMPORAL), LATE's visibility write, LOD selection of the emitted
-// ones, and their staging as (objectId, lodId) after the `run` already staged for the chunk.
-// A survivor is the two words of a Survivor: a = {obj | tags, centre}, b = {r, scale, lodOff, lodCnt}.
-// kModeFrame1 emits the survivors visible last frame (its pass-1 records) and tests no pyramid.
+// The surface table's fields the object stages read, copied into shared memory by each block when the
+// table is small enough; null pointers: read the table in global memory.
+struct SurfaceCache {
+    const float2* bound;  // what the reject test reads: radius, centre norm (see surface_bound)
+    const float4* sphere;
+    const uint2* lod;     // lodOffset, lodCount
+    const float* error;   // every LOD's error, when there are few enough; null: read the LOD table
+};
+
+__device__ __forceinline__ bool lod_range_ok(uint2 lod, uint32_t lodCount) {
+    return lod.x < lodCount && lod.y <= lodCount - lod.x;
+}
+
+// Dense stage over n <= 32 queued objects starting at ring index head, one per lane, in object order:
+// the exact frustum test, where it is not behind them (REJECT); for the objects inside, the sphere projection and Hi-Z test (LATE/TEMPORAL);
+// LATE's visibility write; LOD selection of the emitted ones, and their staging as (objectId, lodId)
+// after the `run` already staged for the chunk.
+// kModeFrame1 emits the survivors visible last frame (its pass-1 records), tests no pyramid and appends
+// every object inside the frustum to the chunk's kept survivors (keep[kept ...], 32 bytes each).
 // The fused modes stage pass 2's records in `stage` and pass 1's in `stage1` (run1).
-template <int MODE>
-__device__ __forceinline__ void dense_entry(const SceneTables& sc, const BatchViewDev& bv, const ViewConsts& v, uint4 a,
-                                            uint4 b, bool mine, uint2* stage, uint32_t& run, uint2* stage1 = nullptr,
-                                            uint32_t* run1 = nullptr, uint32_t* hist = nullptr) {
+template <int MODE, bool REJECT>
+__device__ __forceinline__ void dense_round(const SceneTables& sc, const BatchViewDev& bv, const ViewConsts& v,
+                                            const SurfaceCache& surf, const Ring<REJECT>& ring, uint32_t head, uint32_t n,
+                                            unsigned int& flags, uint2* stage, uint32_t& run, uint4* keep, uint32_t& kept,
+                                            uint2* stage1, uint32_t* run1, uint32_t* hist, uint32_t lt) {
     constexpr bool FUSED = fused_mode(MODE);
     constexpr bool REWRITE = MODE == BLZ_MODE_LATE || FUSED;  // pass 2's visibility rewrite
-    const uint32_t obj = a.x & 0x3FFFFFFFu;  // LATE: bit 31 previous visibility != 0, bit 30 == 1
-    const Vec3 c{__uint_as_float(a.y), __uint_as_float(a.z), __uint_as_float(a.w)};
-    const float r = __uint_as_float(b.x), scale = __uint_as_float(b.y);
-    const bool wasNonZero = (a.x >> 31) != 0u;
-    bool visible = mine;
-    if (mine) {
-        if (MODE == BLZ_MODE_LATE || MODE == BLZ_MODE_TEMPORAL || FUSED) {
-            float4 aabb;
-            if (project_sphere(c, r, v.zNear, v.proj0, v.proj5, aabb))
-                visible = occlusion<MODE == kModeFramePyr>(aabb, bv.pyr, v, c, r);
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t at = (head + lane) & (kRing - 1u);
+    const uint4 ra = ring.a[at], rb = ring.b[at];
+    const bool mine = lane < n;
+    const uint32_t obj = ra.x & 0x3FFFFFFFu, vis = ra.x >> 30;  // (vis: 2 for every word above 1)
+    const bool wasNonZero = vis != 0u;
+    Vec3 c;
+    float r, scale;
+    uint2 lod;
+    bool inside = mine;
+    if constexpr (REJECT) {
+        const uint2 rc = ring.c[at];
+        const bool known = mine && ra.y != kBadObject;
+        const uint32_t sid = known ? ra.y : 0u;
+        float4 sph;
+        if (surf.sphere != nullptr) {
+            sph = surf.sphere[sid];
+            lod = surf.lod[sid];
+        } else {
+            const float4* sp = reinterpret_cast<const float4*>(sc.surfaces + sid);
+            sph = ldp(sp);
+            const uint4 s1 = ldp(reinterpret_cast<const uint4*>(sp + 1));  // materialId, lodOffset, lodCount, vertexOffset
+            lod = make_uint2(s1.y, s1.z);
         }
-        if (REWRITE) {
-            // drawOccLate.cs.hlsl:67, storing only a value that changes
-            const bool wasOne = ((a.x >> 30) & 1u) != 0u;
-            if (visible ? !wasOne : wasNonZero) bv.vis[obj] = visible ? 1u : 0u;
+        const bool good = known && lod_range_ok(lod, sc.lodCount);
+        if (mine && !good) flags |= BLZ_FLAG_BAD_INDEX;
+        const float4 ps = make_float4(__uint_as_float(ra.z), __uint_as_float(ra.w), __uint_as_float(rb.x), __uint_as_float(rb.y));
+        const float4 q = make_float4(__uint_as_float(rb.z), __uint_as_float(rb.w), __uint_as_float(rc.x), __uint_as_float(rc.y));
+        c = view_transform(v.rows, model_to_world(Vec3{sph.x, sph.y, sph.z}, ps, q));
+        r = BLZ_FM(sph.w, ps.w);
+        scale = ps.w;
+        inside = good && frustum_check(c, r, v);
+    } else {
+        c = Vec3{__uint_as_float(ra.y), __uint_as_float(ra.z), __uint_as_float(ra.w)};
+        r = __uint_as_float(rb.x);
+        scale = __uint_as_float(rb.y);
+        lod = make_uint2(rb.z, rb.w);
+    }
+    bool visible = inside;
+    if (inside && (MODE == BLZ_MODE_LATE || MODE == BLZ_MODE_TEMPORAL || FUSED)) {
+        float4 aabb;
+        if (project_sphere(c, r, v.zNear, v.proj0, v.proj5, aabb))
+            visible = occlusion<MODE == kModeFramePyr>(aabb, bv.pyr, v, c, r);
+    }
+    if (MODE == kModeFrame1) {
+        const unsigned k = __ballot_sync(0xFFFFFFFFu, inside);
+        if (inside) {
+            uint4* e = keep + 2u * (kept + __popc(k & lt));
+            const uint32_t tag = (vis != 0u ? 0x80000000u : 0u) | (vis == 1u ? 0x40000000u : 0u);
+            e[0] = make_uint4(obj | tag, __float_as_uint(c.x), __float_as_uint(c.y), __float_as_uint(c.z));
+            e[1] = make_uint4(__float_as_uint(r), __float_as_uint(scale), lod.x, lod.y);
         }
+        kept += __popc(k);
+    } else if (REWRITE && mine) {
+        // drawOccLate.cs.hlsl:67, storing only a value that changes
+        const uint32_t now = visible ? 1u : 0u;
+        if (vis != now) bv.vis[obj] = now;
     }
     // drawOccLate.cs.hlsl:45; a kept frame's pass 1 emits what drawOccFirst.cs.hlsl:22-25 admits
     const bool emitted = visible && (REWRITE ? !wasNonZero : (MODE == kModeFrame1 ? wasNonZero : true));
-    // the fused sweep's pass 1: every survivor visible last frame (its frustum test passed)
-    const bool emitted1 = FUSED && mine && wasNonZero;
+    // the fused sweep's pass 1: every object inside the frustum that was visible last frame
+    const bool emitted1 = FUSED && inside && wasNonZero;
     uint32_t lid = 0u;
     if (emitted || emitted1) {
         // cullBuffers.hlsl:42-55 — last LOD in [1, lodCount) with error < threshold
         const float threshold = lod_threshold(c, r, scale, v.lodTarget);
         uint32_t sel = 0;
-        for (uint32_t t = 1; t < b.w; ++t)
-            if (ldp(&sc.lods[b.z + t].error) < threshold) sel = t;
-        lid = b.z + sel;
+        if (surf.error != nullptr) {
+            for (uint32_t t = 1; t < lod.y; ++t)
+                if (surf.error[lod.x + t] < threshold) sel = t;
+        } else {
+            for (uint32_t t = 1; t < lod.y; ++t)
+                if (ldp(&sc.lods[lod.x + t].error) < threshold) sel = t;
+        }
+        lid = lod.x + sel;
     }
     const unsigned e = __ballot_sync(0xFFFFFFFFu, emitted);
-    if (emitted) stage[run + __popc(e & lanemask_lt())] = make_uint2(obj, lid);
+    if (emitted) stage[run + __popc(e & lt)] = make_uint2(obj, lid);
     run += __popc(e);
     if constexpr (MODE == kModeInstanced) {
         // the group's histogram row (hist = row of this chunk's group): one add per distinct LOD
         const uint32_t idBits = sc.lodCount > 1u ? 32u - static_cast<uint32_t>(__clz(static_cast<int>(sc.lodCount - 1u))) : 0u;
         const unsigned peers = same_lod_lanes(lid, idBits, emitted);
-        if (emitted && (peers & lanemask_lt()) == 0u) atomicAdd(hist + lid, static_cast<uint32_t>(__popc(peers)));
+        if (emitted && (peers & lt) == 0u) atomicAdd(hist + lid, static_cast<uint32_t>(__popc(peers)));
     }
     if constexpr (FUSED) {
         const unsigned e1 = __ballot_sync(0xFFFFFFFFu, emitted1);
-        if (emitted1) stage1[*run1 + __popc(e1 & lanemask_lt())] = make_uint2(obj, lid);
+        if (emitted1) stage1[*run1 + __popc(e1 & lt)] = make_uint2(obj, lid);
         *run1 += __popc(e1);
     }
 }
 
-// dense_entry over n <= 32 queued survivors starting at ring index head. kModeFrame1 also appends
-// them to the chunk's kept survivors (keep[kept ...], 32 bytes each, coalesced).
-template <int MODE>
-__device__ __forceinline__ void dense_round(const SceneTables& sc, const BatchViewDev& bv, const ViewConsts& v,
-                                            const Survivor* ring, uint32_t head, uint32_t n, uint2* stage,
-                                            uint32_t& run, uint4* keep, uint32_t& kept, uint2* stage1, uint32_t* run1,
-                                            uint32_t* hist = nullptr) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const bool mine = lane < n;
-    uint4 a = make_uint4(0u, 0u, 0u, 0u), b = make_uint4(0u, 0u, 0u, 0u);
-    if (mine) {
-        const uint4* e = reinterpret_cast<const uint4*>(ring + ((head + lane) & (kRing - 1u)));
-        a = e[0];
-        b = e[1];
-        if constexpr (MODE == kModeFrame1) {
-            keep[2u * (kept + lane)] = a;
-            keep[2u * (kept + lane) + 1u] = b;
-        }
-    }
-    if constexpr (MODE == kModeFrame1) kept += n;
-    dense_entry<MODE>(sc, bv, v, a, b, mine, stage, run, stage1, run1, hist);
-}
-
-// The fields of the surface table the frustum stage reads (bounding sphere; LOD offset and count),
-// copied into shared memory by each block when the table is small enough; null pointers: read the
-// table in global memory.
-struct SurfaceCache {
-    const float4* sphere;
-    const uint2* lod;
+// A view's constants as a batch's warp keeps them.
+struct SharedView {
+    ViewConsts v;
+    RejectBounds rj;
+    float pad;
 };
+
+// Pass 1's queue of the objects visible last frame (single views; empty in every other kernel), per warp.
+template <uint32_t SLOTS>
+struct Candidates {
+    uint2 ro[SLOTS];
+    uint32_t obj[SLOTS];
+};
+__host__ __device__ constexpr uint32_t candidate_slots(int mode, bool single, int opt) {
+    return mode == BLZ_MODE_FIRST && single ? 2u * 32u * opt : 1u;
+}
 
 // One warp decides the objects [base, limit) of a view, 32 * OPT at a time (object
 // sb + k * 32 + lane for k < OPT, so lanes ascend within each 32-object slice):
-//   1  every lane loads its OPT render objects (fetched one step ahead) and their transforms and
-//      surfaces, and runs the frustum test — without branches: an object that is out of range,
-//      not active in this pass or has a bad id reads the tables' first rows and is masked out.
-//      Pass 1 (single views) first packs the objects visible last frame into a candidate ring,
-//      so the frustum stage runs on full lanes there too;
-//   2  each slice's survivors are appended, in object order, to the warp's ring in shared memory;
+//   1  every lane loads its OPT render objects (fetched one step ahead) and their transforms, and runs
+//      the frustum test (REJECT: drops the objects a bound proves outside, 34 operations against 75)
+//      — without branches: an object that is out of range, not active in this pass or has a bad id reads
+//      the tables' first rows and is masked out (REJECT: or queued). Pass 1 (single views) first packs
+//      the objects visible last frame into a candidate ring, so this stage runs on full lanes there too;
+//   2  what is left of each slice is appended, in object order, to the warp's ring in shared memory;
 //      whenever 32 are waiting they go through the dense stage on full lanes, so the costly part
-//      (projection, Hi-Z, LOD) never runs on a lane without an object;
+//      (REJECT: the exact frustum test; projection, Hi-Z, LOD) never runs on a lane without an object;
 //   3  the dense stage stages the emitted ones in order; the rest drains at the end.
 // Returns the number of records staged. No block barrier: warps never wait for one another.
 template <int MODE, bool SINGLE, int OPT>
 __device__ __forceinline__ uint32_t decide_run_warp(const SceneTables& sc, const BatchViewDev& bv, uint32_t base,
-                                                    uint32_t limit, uint2* stage, Survivor* ring, uint4* cand,
-                                                    const SurfaceCache& surf, unsigned int& flags, uint4* keep,
+                                                    uint32_t limit, uint2* stage, Ring<reject_mode(MODE, SINGLE)>& ring, Candidates<candidate_slots(MODE, SINGLE, OPT)>& cand,
+                                                    const SurfaceCache& surf, SharedView* shared, unsigned int& flags, uint4* keep,
                                                     uint32_t& kept, uint2* stage1 = nullptr, uint32_t* run1 = nullptr,
                                                     const unsigned int* ready = nullptr, uint32_t spinLimit = 0u,
                                                     uint32_t* hist = nullptr) {
     constexpr uint32_t STEP = 32u * OPT;
+    constexpr bool REJECT = reject_mode(MODE, SINGLE);
     constexpr bool PACK = (MODE == BLZ_MODE_FIRST) && SINGLE;  // candidate ring of 2 * STEP entries
     // Single-view pass 2 walks its chunk from the last object down: pass 1 walked the same chunk
     // upwards just before (with only the pyramid build between), so the lines it touched last are
@@ -232,7 +290,7 @@ __device__ __forceinline__ uint32_t decide_run_warp(const SceneTables& sc, const
     constexpr bool DOWN = (MODE == BLZ_MODE_LATE) && SINGLE;
     constexpr uint32_t kNoObject = 0xFFFFFFFFu;
     auto walk = [&](uint32_t i) -> uint32_t { return i < limit ? (DOWN ? base + limit - 1u - i : i) : kNoObject; };
-    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
     if (sc.transformCount == 0u || sc.surfaceCount == 0u) {
         // nothing can be looked up: every object of the pass has a bad id and none is visible
         for (uint32_t i = base + lane; i < limit; i += 32u) {
@@ -242,7 +300,31 @@ __device__ __forceinline__ uint32_t decide_run_warp(const SceneTables& sc, const
         }
         return 0u;
     }
-    const ViewConsts v = load_view(bv.view);
+    // The view's constants: a single view's come from the launch parameters, whose reads are operands of the
+    // arithmetic; a batch's are kept in shared memory by the warp and read again by each step and each
+    // dense round, since together with the loop's state they do not fit the registers.
+    if constexpr (!SINGLE) {
+        __syncwarp();  // the chunk before this one is done with them
+        if (threadIdx.x % 32u == 0u) {
+            shared->v = load_view(bv.view);
+            shared->rj = reject_bounds(shared->v);
+        }
+        __syncwarp();
+    }
+    ViewConsts own;
+    RejectBounds ownRj;
+    if constexpr (SINGLE) {
+        own = load_view(bv.view);
+        ownRj = reject_bounds(own);
+    }
+    const ViewConsts& v = SINGLE ? own : shared->v;
+    [[maybe_unused]] const RejectBounds& rj = SINGLE ? ownRj : shared->rj;
+    // what the loop reads of the view, kept in registers (a batch's views lie in global memory, from where
+    // every field would be read again after each store)
+    const uint2* const objects = reinterpret_cast<const uint2*>(bv.objects);
+    uint32_t* const visWords = bv.vis;
+    const BlzMeshTransform* const dynT = SINGLE ? nullptr : bv.dynT;
+    const uint32_t dynCount = SINGLE || dynT == nullptr ? 0u : bv.dynCount;
     uint32_t run = 0, head = 0, tail = 0;
     // kModeFramePyr: the pyramid is waited for once, before the warp's first dense round
     bool pyrSeen = MODE != kModeFramePyr;
@@ -251,15 +333,17 @@ __device__ __forceinline__ uint32_t decide_run_warp(const SceneTables& sc, const
             wait_pyramid(ready, spinLimit, flags);
             pyrSeen = true;
         }
-        dense_round<MODE>(sc, bv, v, ring, head, n, stage, run, keep, kept, stage1, run1, hist);
+        dense_round<MODE, REJECT>(sc, bv, v, surf, ring, head, n, flags, stage, run, keep, kept, stage1, run1, hist, lt);
     };
 
     // frustum stage over OPT slices: obj[k] the object index, ro[k] its render object, vis[k] the
     // object's visibility word (LATE: as read; the object is active when in range) or, in the other
     // passes, non-zero when the object is active
-    float4 ps[OPT], q[OPT], sph[OPT];
+    float4 ps[OPT], q[OPT];
+    float2 bound[OPT];   // REJECT
+    float4 sph[OPT];     // else
     uint2 lod[OPT];
-    bool ok[OPT];
+    uint32_t sid[OPT];   // or kBadObject
     // LATE and kModeFrame1 test every object (vis[k] holds its visibility word), the others the
     // objects with vis[k] != 0
     constexpr bool ALL = MODE == BLZ_MODE_LATE || MODE == kModeFrame1 || fused_mode(MODE);
@@ -267,22 +351,24 @@ __device__ __forceinline__ uint32_t decide_run_warp(const SceneTables& sc, const
     auto gather = [&](const uint32_t (&obj)[OPT], const uint2 (&ro)[OPT], const uint32_t (&vis)[OPT]) {
 #pragma unroll
         for (int k = 0; k < OPT; ++k) {
-            ok[k] = active(obj[k], vis[k]) && ro[k].x < sc.transformCount && ro[k].y < sc.surfaceCount;
-            const uint32_t tid = ok[k] ? ro[k].x : 0u, sid = ok[k] ? ro[k].y : 0u;
-            if constexpr (!SINGLE) {
-                if (bv.dynT != nullptr && tid < bv.dynCount) {  // the view's own rows first
-                    ldg_transform(bv.dynT + tid, ps[k], q[k]);
+            const bool ok = active(obj[k], vis[k]) && ro[k].x < sc.transformCount && ro[k].y < sc.surfaceCount;
+            const uint32_t tid = ok ? ro[k].x : 0u, s = ok ? ro[k].y : 0u;
+            sid[k] = ok ? s : kBadObject;
+            const BlzMeshTransform* rows = tid < sc.dynCount ? sc.dynRows : sc.transforms;
+            if (!SINGLE && tid < dynCount) rows = dynT;  // the view's own rows first
+            ldg_transform(rows + tid, ps[k], q[k]);
+            const float4* sp = reinterpret_cast<const float4*>(sc.surfaces + s);
+            if constexpr (REJECT) {
+                if (surf.bound != nullptr) {
+                    bound[k] = surf.bound[s];
                 } else {
-                    load_transform(sc, tid, ps[k], q[k]);
+                    const uint4 s1 = ldp(reinterpret_cast<const uint4*>(sp + 1));
+                    bound[k] = surface_bound(ldp(sp), lod_range_ok(make_uint2(s1.y, s1.z), sc.lodCount));
                 }
+            } else if (surf.sphere != nullptr) {
+                sph[k] = surf.sphere[s];
+                lod[k] = surf.lod[s];
             } else {
-                load_transform(sc, tid, ps[k], q[k]);
-            }
-            if (surf.sphere != nullptr) {
-                sph[k] = surf.sphere[sid];
-                lod[k] = surf.lod[sid];
-            } else {
-                const float4* sp = reinterpret_cast<const float4*>(sc.surfaces + sid);
                 sph[k] = ldp(sp);
                 const uint4 s1 = ldp(reinterpret_cast<const uint4*>(sp + 1));  // materialId, lodOffset, lodCount, vertexOffset
                 lod[k] = make_uint2(s1.y, s1.z);
@@ -293,20 +379,32 @@ __device__ __forceinline__ uint32_t decide_run_warp(const SceneTables& sc, const
 #pragma unroll
         for (int k = 0; k < OPT; ++k) {
             const bool act = active(obj[k], vis[k]);
-            const bool lodOk = lod[k].x < sc.lodCount && lod[k].y <= sc.lodCount - lod[k].x;
-            const bool good = ok[k] && lodOk;
-            if (act && !good) flags |= BLZ_FLAG_BAD_INDEX;
-            const Vec3 c = view_transform(v.rows, model_to_world(Vec3{sph[k].x, sph[k].y, sph[k].z}, ps[k], q[k]));
-            const float r = BLZ_FM(sph[k].w, ps[k].w);
-            const bool inFrustum = good && frustum_check(c, r, v);
+            bool queued;
+            Vec3 c{0.f, 0.f, 0.f};
+            float r = 0.f;
+            if constexpr (REJECT) {
+                queued = act && (sid[k] == kBadObject || !surely_outside(ps[k], q[k], bound[k], v, rj));
+            } else {
+                const bool good = sid[k] != kBadObject && lod_range_ok(lod[k], sc.lodCount);
+                if (act && !good) flags |= BLZ_FLAG_BAD_INDEX;
+                c = view_transform(v.rows, model_to_world(Vec3{sph[k].x, sph[k].y, sph[k].z}, ps[k], q[k]));
+                r = BLZ_FM(sph[k].w, ps[k].w);
+                queued = good && frustum_check(c, r, v);
+            }
             // drawOccLate.cs.hlsl:67, storing only a value that changes
-            if (ALL && act && !inFrustum && vis[k] != 0u) bv.vis[obj[k]] = 0u;
-            const unsigned m = __ballot_sync(0xFFFFFFFFu, inFrustum);
-            if (inFrustum) {
-                uint4* e = reinterpret_cast<uint4*>(ring + ((tail + __popc(m & lanemask_lt())) & (kRing - 1u)));
-                const uint32_t tag = !ALL ? 0u : (vis[k] != 0u ? 0x80000000u : 0u) | (vis[k] == 1u ? 0x40000000u : 0u);
-                e[0] = make_uint4(obj[k] | tag, __float_as_uint(c.x), __float_as_uint(c.y), __float_as_uint(c.z));
-                e[1] = make_uint4(__float_as_uint(r), __float_as_uint(ps[k].w), lod[k].x, lod[k].y);
+            if (ALL && act && !queued && vis[k] != 0u) visWords[obj[k]] = 0u;
+            const unsigned m = __ballot_sync(0xFFFFFFFFu, queued);
+            if (queued) {
+                const uint32_t at = (tail + __popc(m & lt)) & (kRing - 1u);
+                const uint32_t o = obj[k] | (ALL ? min(vis[k], 2u) << 30 : 0u);
+                if constexpr (REJECT) {
+                    ring.a[at] = make_uint4(o, sid[k], __float_as_uint(ps[k].x), __float_as_uint(ps[k].y));
+                    ring.b[at] = make_uint4(__float_as_uint(ps[k].z), __float_as_uint(ps[k].w), __float_as_uint(q[k].x), __float_as_uint(q[k].y));
+                    ring.c[at] = make_uint2(__float_as_uint(q[k].z), __float_as_uint(q[k].w));
+                } else {
+                    ring.a[at] = make_uint4(o, __float_as_uint(c.x), __float_as_uint(c.y), __float_as_uint(c.z));
+                    ring.b[at] = make_uint4(__float_as_uint(r), __float_as_uint(ps[k].w), lod[k].x, lod[k].y);
+                }
             }
             tail += __popc(m);
             if (tail - head >= 32u) {
@@ -325,10 +423,10 @@ __device__ __forceinline__ uint32_t decide_run_warp(const SceneTables& sc, const
         for (int k = 0; k < OPT; ++k) {
             const uint32_t i = walk(at + k * 32u + lane);
             const bool in = i != kNoObject;
-            nro[k] = in ? ldp(reinterpret_cast<const uint2*>(bv.objects) + i) : make_uint2(0u, 0u);
+            nro[k] = in ? ldp(objects + i) : make_uint2(0u, 0u);
             nvis[k] = in ? 1u : 0u;
-            if (MODE == BLZ_MODE_FIRST && in) nvis[k] = ldp(bv.vis + i);
-            if (ALL) nvis[k] = in ? bv.vis[i] : 0u;  // rewritten later by this warp: coherent load
+            if (MODE == BLZ_MODE_FIRST && in) nvis[k] = ldp(visWords + i);
+            if (ALL) nvis[k] = in ? visWords[i] : 0u;
         }
     };
     // candidates packed by pass 1, taken STEP at a time (or the rest, at the end)
@@ -340,10 +438,10 @@ __device__ __forceinline__ uint32_t decide_run_warp(const SceneTables& sc, const
 #pragma unroll
         for (int k = 0; k < OPT; ++k) {
             const uint32_t j = k * 32u + lane;
-            const uint4 e = cand[(ahead + j) & (2u * STEP - 1u)];
+            const uint32_t at = (ahead + j) & (2u * STEP - 1u);
             const bool in = j < n;
-            obj[k] = e.x;
-            ro[k] = make_uint2(e.y, e.z);
+            obj[k] = cand.obj[at];
+            ro[k] = cand.ro[at];
             vis[k] = in ? 1u : 0u;
         }
         __syncwarp();
@@ -368,7 +466,11 @@ __device__ __forceinline__ uint32_t decide_run_warp(const SceneTables& sc, const
             for (int k = 0; k < OPT; ++k) {
                 const bool act = vis[k] != 0u;
                 const unsigned m = __ballot_sync(0xFFFFFFFFu, act);
-                if (act) cand[(atail + __popc(m & lanemask_lt())) & (2u * STEP - 1u)] = make_uint4(obj[k], ro[k].x, ro[k].y, 0u);
+                if (act) {
+                    const uint32_t at = (atail + __popc(m & lt)) & (2u * STEP - 1u);
+                    cand.obj[at] = obj[k];
+                    cand.ro[at] = ro[k];
+                }
                 atail += __popc(m);
             }
             if (atail - ahead >= STEP) take_candidates(STEP);
@@ -407,19 +509,26 @@ __device__ __forceinline__ void put_record(uint8_t* cmds, uint32_t stride, uint3
 
 // ------------------------------------------------------------------ decide kernel
 
-// Shared memory of the decide kernels: one survivor ring per warp, pass 1's candidate rings, and the
-// surface table in what static shared memory is left (48 KB per block).
+// Shared memory of the decide kernels: one ring per warp, pass 1's candidate rings, and the surface
+// table in what static shared memory is left (48 KB per block).
 template <int MODE, bool SINGLE, int THREADS, int OPT>
 struct DecideSmem {
     static constexpr int NW = THREADS / 32;
-    static constexpr bool PACK = (MODE == BLZ_MODE_FIRST) && SINGLE;
-    static constexpr size_t kUsed = sizeof(Survivor) * kRing * NW + (PACK ? sizeof(uint4) * NW * 2 * 32 * OPT : 0);
-    static constexpr size_t kLeft = kUsed + 1024 < 48 * 1024 ? 48 * 1024 - 1024 - kUsed : 0;
-    static constexpr uint32_t kSurf = kLeft >= 512 * 24 ? 512u : (kLeft >= 256 * 24 ? 256u : (kLeft >= 64 * 24 ? 64u : 1u));
-    Survivor ring[NW][kRing];
-    uint4 cand[PACK ? NW : 1][PACK ? 2 * 32 * OPT : 1];
+    using Cand = Candidates<candidate_slots(MODE, SINGLE, OPT)>;
+    using Queue = Ring<reject_mode(MODE, SINGLE)>;
+    static constexpr size_t kUsed = (sizeof(Queue) + sizeof(Cand) + (SINGLE ? 0 : sizeof(SharedView))) * NW + sizeof(SharedView);
+    static constexpr bool REJECT = reject_mode(MODE, SINGLE);
+    static constexpr uint32_t kLods = REJECT && kUsed + 2048 + 1024 <= 48 * 1024 ? 512u : 1u;  // LOD errors
+    static constexpr size_t kLeft = kUsed + kLods * 4 + 1024 < 48 * 1024 ? 48 * 1024 - 1024 - kLods * 4 - kUsed : 0;
+    static constexpr size_t kSurfBytes = (REJECT ? sizeof(float2) : 0) + sizeof(float4) + sizeof(uint2);
+    static constexpr uint32_t kSurf = kLeft >= 512 * kSurfBytes ? 512u : (kLeft >= 256 * kSurfBytes ? 256u : (kLeft >= 64 * kSurfBytes ? 64u : 1u));
+    Queue ring[NW];
+    SharedView view[SINGLE ? 1 : NW];
+    Cand cand[NW];
     float4 sphere[kSurf];
+    float2 bound[REJECT ? kSurf : 1u];
     uint2 lod[kSurf];
+    float error[kLods];
 };
 
 // The decide kernels' body: each warp decides chunks of a view (decide_run_warp) and records each
@@ -429,19 +538,25 @@ __device__ __forceinline__ void decide_body(const PipeParams& p, DecideSmem<MODE
                                             const unsigned int* ready = nullptr, uint32_t spinLimit = 0u) {
     using Smem = DecideSmem<MODE, SINGLE, THREADS, OPT>;
     constexpr int NW = Smem::NW;
-    constexpr bool PACK = Smem::PACK;
     constexpr uint32_t kSurf = Smem::kSurf;
-    SurfaceCache surf{nullptr, nullptr};
+    SurfaceCache surf{nullptr, nullptr, nullptr, nullptr};
+    if (Smem::kLods > 1u && p.sc.lodCount <= Smem::kLods) {
+        for (uint32_t i = threadIdx.x; i < p.sc.lodCount; i += THREADS) sm.error[i] = ldp(&p.sc.lods[i].error);
+        surf.error = sm.error;
+    }
     if (kSurf > 1u && p.sc.surfaceCount <= kSurf) {
         for (uint32_t i = threadIdx.x; i < p.sc.surfaceCount; i += THREADS) {
             const float4* sp = reinterpret_cast<const float4*>(p.sc.surfaces + i);
-            sm.sphere[i] = ldp(sp);
-            const uint4 s1 = ldp(reinterpret_cast<const uint4*>(sp + 1));
-            sm.lod[i] = make_uint2(s1.y, s1.z);
+            const float4 sph = ldp(sp);
+            const uint4 s1 = ldp(reinterpret_cast<const uint4*>(sp + 1));  // materialId, lodOffset, lodCount, vertexOffset
+            const uint2 lod = make_uint2(s1.y, s1.z);
+            sm.sphere[i] = sph;
+            if (Smem::REJECT) sm.bound[i] = surface_bound(sph, lod_range_ok(lod, p.sc.lodCount));
+            sm.lod[i] = lod;
         }
-        __syncthreads();
-        surf = SurfaceCache{sm.sphere, sm.lod};
+        surf = SurfaceCache{sm.bound, sm.sphere, sm.lod, surf.error};
     }
+    __syncthreads();
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t warpsTotal = gridDim.x * NW;
     const uint32_t chunkSize = p.chunkSize;
@@ -455,9 +570,10 @@ __device__ __forceinline__ void decide_body(const PipeParams& p, DecideSmem<MODE
         if (lane == 0) c = warpsTotal + atomicAdd(p.workCounter, 1u);
         return __shfl_sync(0xFFFFFFFFu, c, 0);
     };
-    uint32_t chunk = blockIdx.x * NW + warp;
-    while (chunk < p.totalTiles) {
-        const uint32_t next = next_chunk(chunk);  // asked now, used after this chunk
+    uint32_t item = blockIdx.x * NW + warp;
+    while (item < p.totalTiles) {
+        const uint32_t next = next_chunk(item);  // asked now, used after this chunk
+        const uint32_t chunk = !SINGLE && p.order != nullptr ? __ldcg(p.order + item) : item;
         uint32_t vi = 0, first = 0;
         if constexpr (!SINGLE) {
             vi = find_view_warp(p.tileStart, p.viewCount, chunk);
@@ -467,24 +583,25 @@ __device__ __forceinline__ void decide_body(const PipeParams& p, DecideSmem<MODE
         const uint32_t base = (chunk - first) * chunkSize;
         const uint32_t limit = min(base + chunkSize, bv.count);
         uint2* stage = p.staged + static_cast<size_t>(chunk) * chunkSize;
-        Survivor* ring = sm.ring[warp];
-        uint4* cand = sm.cand[PACK ? warp : 0];
+        auto& ring = sm.ring[warp];
+        auto& cand = sm.cand[warp];
+        SharedView* shared = &sm.view[SINGLE ? 0u : warp];
         uint32_t total = 0, kept = 0, total1 = 0;
         uint4* keep = nullptr;
         if constexpr (MODE == kModeFrame1) keep = static_cast<uint4*>(p.keep) + 2u * static_cast<size_t>(chunk) * chunkSize;
         uint2* stage1 = nullptr;
         if constexpr (fused_mode(MODE)) stage1 = p.staged2 + static_cast<size_t>(chunk) * chunkSize;
-        if (MODE == kModeRuntime) {
+        if constexpr (MODE == kModeRuntime) {
             switch (bv.mode) {
-                case BLZ_MODE_FIRST: total = decide_run_warp<BLZ_MODE_FIRST, SINGLE, OPT>(p.sc, bv, base, limit, stage, ring, cand, surf, flags, keep, kept); break;
-                case BLZ_MODE_LATE: total = decide_run_warp<BLZ_MODE_LATE, SINGLE, OPT>(p.sc, bv, base, limit, stage, ring, cand, surf, flags, keep, kept); break;
-                case BLZ_MODE_TEMPORAL: total = decide_run_warp<BLZ_MODE_TEMPORAL, SINGLE, OPT>(p.sc, bv, base, limit, stage, ring, cand, surf, flags, keep, kept); break;
-                default: total = decide_run_warp<BLZ_MODE_FRUSTUM, SINGLE, OPT>(p.sc, bv, base, limit, stage, ring, cand, surf, flags, keep, kept); break;
+                case BLZ_MODE_FIRST: total = decide_run_warp<BLZ_MODE_FIRST, SINGLE, OPT>(p.sc, bv, base, limit, stage, ring, cand, surf, shared, flags, keep, kept); break;
+                case BLZ_MODE_LATE: total = decide_run_warp<BLZ_MODE_LATE, SINGLE, OPT>(p.sc, bv, base, limit, stage, ring, cand, surf, shared, flags, keep, kept); break;
+                case BLZ_MODE_TEMPORAL: total = decide_run_warp<BLZ_MODE_TEMPORAL, SINGLE, OPT>(p.sc, bv, base, limit, stage, ring, cand, surf, shared, flags, keep, kept); break;
+                default: total = decide_run_warp<BLZ_MODE_FRUSTUM, SINGLE, OPT>(p.sc, bv, base, limit, stage, ring, cand, surf, shared, flags, keep, kept); break;
             }
         } else {
             uint32_t* hist = nullptr;
             if constexpr (MODE == kModeInstanced) hist = p.instHist + static_cast<size_t>(chunk / kInstGroup) * p.instLods;
-            total = decide_run_warp<(MODE < 0 ? 0 : MODE), SINGLE, OPT>(p.sc, bv, base, limit, stage, ring, cand, surf, flags, keep, kept,
+            total = decide_run_warp<(MODE < 0 ? 0 : MODE), SINGLE, OPT>(p.sc, bv, base, limit, stage, ring, cand, surf, shared, flags, keep, kept,
                                                                        stage1, &total1, ready, spinLimit, hist);
         }
         if (lane == 0) {
@@ -492,13 +609,13 @@ __device__ __forceinline__ void decide_body(const PipeParams& p, DecideSmem<MODE
             if constexpr (MODE == kModeFrame1) p.keepCount[chunk] = kept;
             if constexpr (fused_mode(MODE)) p.chunkCount2[chunk] = total1;
         }
-        chunk = next;
+        item = next;
     }
     if (flags) atomicOr(&p.scratch->status, flags);
 }
 
 template <int MODE, bool SINGLE, int THREADS, int OPT>
-__global__ void __launch_bounds__(THREADS, (SINGLE || MODE >= 0) ? 1024 / THREADS : 1) cull_decide_kernel(const PipeParams p) {
+__global__ void __launch_bounds__(THREADS, SINGLE || MODE >= 0 ? 1024 / THREADS : 1) cull_decide_kernel(const PipeParams p) {
     __shared__ DecideSmem<MODE, SINGLE, THREADS, OPT> sm;
     pdl_wait();
     decide_body<MODE, SINGLE, THREADS, OPT>(p, sm);
@@ -518,7 +635,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) cull_frame_kernel(con
     using Smem = DecideSmem<kModeFramePyr, true, THREADS, OPT>;
     __shared__ Smem sm;
     static_assert(sizeof(sm.ring) >= sizeof(float) * (kPyrSmemA + kPyrSmemB), "the tile buffers live in the rings");
-    float* sA = reinterpret_cast<float*>(&sm.ring[0][0]);
+    float* sA = reinterpret_cast<float*>(&sm.ring[0]);
     float* sB = sA + kPyrSmemA;
     __shared__ uint32_t s_tile;
     pdl_wait();
@@ -539,36 +656,30 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) cull_frame_kernel(con
 
 // ------------------------------------------------------------------ scatter kernel
 
-// Each block owns 32 consecutive chunks, one per warp, and finds where their records go without
-// any grid-wide step: it sums the counts of its first chunk's view that precede that chunk (a
-// strided read of at most one view's counts, from L2), and warp 0 scans the 32 chunks' counts
-// (restarting at view boundaries). The block's warps then copy the chunks' staged records to their slots as full
-// records, and the lane holding a view's last chunk writes that view's draw count. Block 0 also
-// rewinds the decide kernel's work counter for the next launch.
+// Single views. Each block owns 32 consecutive chunks, one per warp, and finds where their records go
+// without any grid-wide step: it sums the counts that precede its first chunk (a strided read of the counts,
+// from L2), and warp 0 scans the 32 chunks' counts. The block's warps then copy the chunks' staged records
+// to their slots as full records, and the lane holding the last chunk writes the draw count.
 constexpr int kScatterWarps = 32;  // one warp per chunk
 constexpr uint32_t kScatterChunks = 32;
 constexpr uint32_t kScatterPre = 3;  // 32-record slices of its chunk a warp loads before the offsets are known
 
-template <bool SINGLE>
 __device__ __forceinline__ void scatter_block(const PipeParams& p, const uint32_t block) {
     __shared__ uint32_t s_part[kScatterWarps];
-    __shared__ uint32_t s_base[kScatterChunks], s_n[kScatterChunks], s_vi[kScatterChunks];
+    __shared__ uint32_t s_base[kScatterChunks], s_n[kScatterChunks];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t chunkSize = p.chunkSize;
     const uint32_t c0 = block * kScatterChunks;
-    if (block == 0 && threadIdx.x == 0 && p.workCounter != nullptr) *p.workCounter = 0u;
     if (c0 >= p.totalTiles) return;
-    const uint32_t vi0 = SINGLE ? 0u : find_view_warp(p.tileStart, p.viewCount, c0);
-    const uint32_t viewStart0 = SINGLE ? 0u : ldp(p.tileStart + vi0);
     // 0. each warp fetches its chunk's count (handed to warp 0 through shared memory) and, once it
     //    is known, its first kScatterPre * 32 staged records, which arrive while the block scans;
     //    their LODs are fetched after the barrier
     const uint32_t myChunk = c0 + warp;
     const uint32_t myN = myChunk < p.totalTiles ? __ldcg(p.chunkCount + myChunk) : 0u;
     const uint2* myStage = p.staged + static_cast<size_t>(myChunk) * chunkSize;
-    // 1. records of the first chunk's view before c0, loaded while the count is on its way
+    // 1. records before c0, loaded while the count is on its way
     uint32_t part = 0;
-    for (uint32_t c = viewStart0 + threadIdx.x; c < c0; c += 8u * kScatterWarps * 32u) {
+    for (uint32_t c = threadIdx.x; c < c0; c += 8u * kScatterWarps * 32u) {
         uint32_t x[8];  // eight loads in flight per thread
 #pragma unroll
         for (uint32_t k = 0; k < 8u; ++k) {
@@ -596,52 +707,23 @@ __device__ __forceinline__ void scatter_block(const PipeParams& p, const uint32_
         const uint32_t i = lane + 32u * u;
         preLod[u] = i < myN ? ldp(reinterpret_cast<const uint2*>(p.sc.lods + pre[u].y)) : make_uint2(0u, 0u);
     }
-    // 2. warp 0: exclusive offsets of the block's chunks, a scan restarting at each view's first chunk
+    // 2. warp 0: exclusive offsets of the block's chunks
     if (warp == 0) {
         uint32_t carry = 0;
 #pragma unroll
         for (int w = 0; w < kScatterWarps; ++w) carry += s_part[w];
-        const uint32_t c = c0 + lane;
-        const bool in = c < p.totalTiles;
         const uint32_t n = s_n[lane];  // 0 past the last chunk
-        uint32_t vi = vi0;
-        bool starts = false;  // this chunk starts a view (the scan restarts here)
-        if constexpr (!SINGLE) {
-            // the next 32 view starts after vi0: a lane's view is vi0 + those at or before its chunk
-            const uint32_t j = vi0 + 1u + lane;
-            const uint32_t sj = j < p.viewCount ? ldp(p.tileStart + j) : 0xFFFFFFFFu;
-            uint32_t cnt = 0;
-#pragma unroll
-            for (int t = 0; t < 32; ++t) cnt += __shfl_sync(0xFFFFFFFFu, sj, t) <= c ? 1u : 0u;
-            if (in) {
-                // more than 32 views (empty ones) can start inside the block's chunks: search then
-                vi = cnt < 32u ? vi0 + cnt : find_view(p.tileStart, p.viewCount, c);
-                starts = c == ldp(p.tileStart + vi);
-            }
-        }
-        // segmented inclusive scan: combine(a, b) = b.starts ? b : a + b
         uint32_t sum = n;
-        bool flag = starts;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t ps = __shfl_up_sync(0xFFFFFFFFu, sum, o);
-            const bool pf = __shfl_up_sync(0xFFFFFFFFu, flag ? 1u : 0u, o) != 0u;
-            if (lane >= static_cast<uint32_t>(o) && !flag) {
-                sum += ps;
-                flag = pf;
-            }
+            if (lane >= static_cast<uint32_t>(o)) sum += ps;
         }
-        // lanes still in the first view (no start at or before them) add the view's earlier records
-        const uint32_t excl = sum - n + (flag ? 0u : carry);
+        const uint32_t excl = carry + sum - n;
         s_base[lane] = excl;
-        s_vi[lane] = vi;
-        if (in) {
-            const bool lastOfView = SINGLE ? (c + 1 == p.totalTiles) : (c + 1 == ldp(p.tileStart + vi + 1));
-            if (lastOfView) {
-                const BatchViewDev& bv = view_of<SINGLE>(p, vi);
-                *bv.drawCount = excl + n;
-                if (excl + n > bv.capacity) atomicOr(&p.scratch->status, BLZ_FLAG_COMMAND_OVERFLOW);
-            }
+        if (c0 + lane + 1u == p.totalTiles) {
+            *p.single.drawCount = excl + n;
+            if (excl + n > p.single.capacity) atomicOr(&p.scratch->status, BLZ_FLAG_COMMAND_OVERFLOW);
         }
     }
     __syncthreads();
@@ -649,9 +731,9 @@ __device__ __forceinline__ void scatter_block(const PipeParams& p, const uint32_
     static_assert(kScatterWarps == static_cast<int>(kScatterChunks), "one warp per chunk");
     if (myChunk >= p.totalTiles) return;
     const uint32_t base = s_base[warp];
-    const BatchViewDev& bv = view_of<SINGLE>(p, s_vi[warp]);
+    const BatchViewDev& bv = p.single;
     // staged record i goes to slot base + i, or base + n - 1 - i for a chunk staged last object first
-    const bool down = SINGLE && p.descending != 0u;
+    const bool down = p.descending != 0u;
 #pragma unroll
     for (uint32_t u = 0; u < kScatterPre; ++u) {
         const uint32_t i = lane + 32u * u;
@@ -670,10 +752,146 @@ __device__ __forceinline__ void scatter_block(const PipeParams& p, const uint32_
     }
 }
 
-template <bool SINGLE>
 __global__ void __launch_bounds__(kScatterWarps * 32, 2) cull_scatter_kernel(const PipeParams p) {
     pdl_wait();
-    scatter_block<SINGLE>(p, blockIdx.x);
+    scatter_block(p, blockIdx.x);
+}
+
+// Batched views: two launches. The scan has a block per view: it scans the counts of the view's chunks into
+// {offset in the view's records, view} per chunk and writes the view's draw count (block 0 also rewinds the
+// decide kernel's work counter). The scatter then is one warp per chunk with nothing to wait for. (One launch
+// of 1024-thread blocks, each finding its chunks' views and offsets behind two barriers, took 23 to 30 us for
+// the 33,000 chunks of the 64-view batch, 3.4 waves of them; the two take 3.6 and 14.)
+constexpr uint32_t kBatchScanThreads = 512, kBatchScanEach = 8;
+constexpr uint32_t kBatchScatterThreads = 256, kBatchScatterChunks = 4;
+
+__global__ void __launch_bounds__(kBatchScanThreads) batch_scan_kernel(const PipeParams p) {
+    constexpr uint32_t NW = kBatchScanThreads / 32u;
+    static_assert(NW <= 32u, "a lane per warp");
+    __shared__ uint32_t s_warp[kBatchScanEach][NW];
+    pdl_wait();
+    const uint32_t vi = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t first = ldp(p.tileStart + vi), end = ldp(p.tileStart + vi + 1u);
+    if (vi == 0u && threadIdx.x == 0u && p.workCounter != nullptr) *p.workCounter = 0u;
+    uint32_t carry = 0;
+    for (uint32_t c0 = first; c0 < end; c0 += kBatchScanThreads * kBatchScanEach) {
+        // thread t takes chunks c0 + t, c0 + t + T, ...: their counts loaded together, T of them scanned at a time
+        uint32_t n[kBatchScanEach], sum[kBatchScanEach];
+#pragma unroll
+        for (uint32_t k = 0; k < kBatchScanEach; ++k) {
+            const uint32_t c = c0 + k * kBatchScanThreads + threadIdx.x;
+            n[k] = c < end ? __ldcg(p.chunkCount + c) : 0u;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kBatchScanEach; ++k) {
+            sum[k] = n[k];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, sum[k], o);
+                if (lane >= static_cast<uint32_t>(o)) sum[k] += x;
+            }
+            if (lane == 31u) s_warp[k][warp] = sum[k];
+        }
+        __syncthreads();
+        // a warp's total before it, over the parts and warps in order
+#pragma unroll
+        for (uint32_t k = 0; k < kBatchScanEach; ++k) {
+            const uint32_t x = lane < NW ? s_warp[k][lane] : 0u;
+            const uint32_t before = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? x : 0u);
+            const uint32_t c = c0 + k * kBatchScanThreads + threadIdx.x;
+            if (c < end) p.chunkBase[c] = make_uint2(carry + before + sum[k] - n[k], vi);
+            carry += __reduce_add_sync(0xFFFFFFFFu, x);
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0u) {
+        const BatchViewDev& bv = p.views[vi];
+        *bv.drawCount = carry;
+        if (carry > bv.capacity) atomicOr(&p.scratch->status, BLZ_FLAG_COMMAND_OVERFLOW);
+    }
+}
+
+__global__ void __launch_bounds__(kBatchScatterThreads) batch_scatter_kernel(const PipeParams p) {
+    constexpr uint32_t CH = kBatchScatterChunks;
+    pdl_wait();
+    const uint32_t lane = threadIdx.x & 31u, c0 = (blockIdx.x * (kBatchScatterThreads / 32u) + (threadIdx.x >> 5)) * CH;
+    // lane k < CH holds chunk c0 + k: its count, its records' first slot, its view
+    const bool has = lane < CH && c0 + lane < p.totalTiles;
+    const uint32_t n = has ? __ldcg(p.chunkCount + c0 + lane) : 0u;
+    const uint2 at = has ? __ldcg(p.chunkBase + c0 + lane) : make_uint2(0u, 0u);
+    uint32_t start[CH + 1u];  // the warp's records run through its chunks in order
+    start[0] = 0u;
+#pragma unroll
+    for (uint32_t k = 0; k < CH; ++k) start[k + 1u] = start[k] + __shfl_sync(0xFFFFFFFFu, n, static_cast<int>(k));
+    const uint32_t total = start[CH];
+    for (uint32_t j0 = 0; j0 < total; j0 += 64u) {  // two records a lane, their loads together
+        uint2 rec[2], lod[2];
+        uint32_t slot[2], vi[2];
+#pragma unroll
+        for (uint32_t u = 0; u < 2u; ++u) {
+            const uint32_t j = j0 + 32u * u + lane;
+            uint32_t k = 0, from = 0;
+#pragma unroll
+            for (uint32_t t = 1; t < CH; ++t)
+                if (j >= start[t]) k = t, from = start[t];
+            slot[u] = __shfl_sync(0xFFFFFFFFu, at.x, static_cast<int>(k)) + (j - from);
+            vi[u] = __shfl_sync(0xFFFFFFFFu, at.y, static_cast<int>(k));
+            rec[u] = j < total ? __ldcg(p.staged + static_cast<size_t>(c0 + k) * p.chunkSize + (j - from)) : make_uint2(0u, 0u);
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 2u; ++u)
+            lod[u] = j0 + 32u * u + lane < total ? ldp(reinterpret_cast<const uint2*>(p.sc.lods + rec[u].y)) : make_uint2(0u, 0u);
+#pragma unroll
+        for (uint32_t u = 0; u < 2u; ++u) {
+            if (j0 + 32u * u + lane >= total) continue;
+            const BatchViewDev& bv = p.views[vi[u]];
+            if (slot[u] < bv.capacity) put_record(bv.cmds, bv.stride, slot[u], rec[u].x, lod[u].x, lod[u].y);
+        }
+    }
+}
+
+constexpr uint32_t kBatchOrderThreads = 64;
+
+// The order in which a batch's chunks are decided: by their place in their view, order[k] = the chunk that
+// comes k-th when the middle of chunk r of a view of R chunks counts as (2r + 1) / 2R, and equal ones go by
+// view. A render list that follows the scene's order then reads the same transform rows at the same time as
+// every other, so the table comes from memory once and not once per view. Exact integers: chunk (v, r) comes
+// after the chunks r' of view u with (2r' + 1) R_v < (2r + 1) R_u, or equal and u < v.
+__global__ void __launch_bounds__(kBatchOrderThreads) batch_order_kernel(const uint32_t* tileStart, uint32_t viewCount, uint32_t total,
+                                                                         uint32_t small, uint32_t* order) {
+    __shared__ uint32_t s_start[kBatchOrderViews + 1u];
+    pdl_wait();
+    for (uint32_t i = threadIdx.x; i <= viewCount; i += kBatchOrderThreads) s_start[i] = ldp(tileStart + i);
+    __syncthreads();
+    const uint32_t c = blockIdx.x * kBatchOrderThreads + threadIdx.x;
+    if (c >= total) return;
+    uint32_t v = 0, hi = viewCount;
+    while (hi - v > 1u) {
+        const uint32_t mid = (v + hi) >> 1;
+        if (s_start[mid] <= c) v = mid;
+        else hi = mid;
+    }
+    const uint32_t Rv = s_start[v + 1u] - s_start[v], odd = 2u * (c - s_start[v]) + 1u;
+    uint32_t rank = 0;
+    if (small) {
+        // fewer than 2^15 chunks a view: (2r + 1) R_u stays below 2^31 and its quotient by R_v below 2^16, so the
+        // quotient from a float reciprocal is at most one off
+        const float inv = 1.0f / static_cast<float>(Rv);
+#pragma unroll 4
+        for (uint32_t u = 0; u < viewCount; ++u) {
+            const uint32_t a = odd * (s_start[u + 1u] - s_start[u]) - (u < v ? 0u : 1u);
+            uint32_t m = static_cast<uint32_t>(static_cast<float>(a) * inv);
+            const int rest = static_cast<int>(a - m * Rv);
+            m = rest < 0 ? m - 1u : (rest >= static_cast<int>(Rv) ? m + 1u : m);
+            rank += (m + 1u) >> 1;
+        }
+    } else {
+        for (uint32_t u = 0; u < viewCount; ++u) {
+            const uint64_t a = static_cast<uint64_t>(odd) * (s_start[u + 1u] - s_start[u]) - (u < v ? 0u : 1u);
+            rank += (static_cast<uint32_t>(a / Rv) + 1u) >> 1;
+        }
+    }
+    order[rank] = c;
 }
 
 // Both record lists of a one-call frame in one launch: blocks [0, blocks1) scatter list 1, the rest
@@ -687,8 +905,8 @@ __global__ void __launch_bounds__(kScatterWarps * 32, 2) cull_scatter2_kernel(co
         p1.scratch->frameTilesDone = 0u;
         p1.scratch->frameReady = 0u;
     }
-    if (blockIdx.x < blocks1) scatter_block<true>(p1, blockIdx.x);
-    else scatter_block<true>(p2, blockIdx.x - blocks1);
+    if (blockIdx.x < blocks1) scatter_block(p1, blockIdx.x);
+    else scatter_block(p2, blockIdx.x - blocks1);
 }
 
 // ------------------------------------------------------------------ kept frame, pass 2
@@ -806,16 +1024,28 @@ template <int MODE, bool SINGLE, int THREADS, int OPT>
 static cudaError_t launch_t(const PipeParams& p, uint32_t blocksPerSm, int smCount, cudaStream_t s) {
     cudaError_t e = launch_decide_t<MODE, SINGLE, THREADS, OPT>(p, blocksPerSm, smCount, s);
     if (e != cudaSuccess) return e;
-    return launch_pdl(cull_scatter_kernel<SINGLE>, scatter_blocks(p), kScatterWarps * 32, 0, s, p);
+    if constexpr (SINGLE) {
+        return launch_pdl(cull_scatter_kernel, scatter_blocks(p), kScatterWarps * 32, 0, s, p);
+    } else {
+        e = launch_pdl(batch_scan_kernel, p.viewCount, kBatchScanThreads, 0, s, p);
+        if (e != cudaSuccess) return e;
+        constexpr uint32_t per = kBatchScatterThreads / 32u * kBatchScatterChunks;
+        return launch_pdl(batch_scatter_kernel, (p.totalTiles + per - 1u) / per, kBatchScatterThreads, 0, s, p);
+    }
 }
 
 uint32_t object_tile_size() { return kChunk; }
+
+cudaError_t launch_batch_order(const PipeParams& p, uint32_t largest, uint32_t* order, cudaStream_t s) {
+    return launch_pdl(batch_order_kernel, (p.totalTiles + kBatchOrderThreads - 1u) / kBatchOrderThreads, kBatchOrderThreads, 0, s, p.tileStart, p.viewCount, p.totalTiles,
+                      largest < (1u << 15) ? 1u : 0u, order);
+}
 
 template <int THREADS, int OPT>
 static cudaError_t launch_frame_first_t(const PipeParams& p, int smCount, cudaStream_t s, bool scatter) {
     cudaError_t e = launch_decide_t<kModeFrame1, true, THREADS, OPT>(p, 0, smCount, s);
     if (e != cudaSuccess || !scatter) return e;
-    return launch_pdl(cull_scatter_kernel<true>, scatter_blocks(p), kScatterWarps * 32, 0, s, p);
+    return launch_pdl(cull_scatter_kernel, scatter_blocks(p), kScatterWarps * 32, 0, s, p);
 }
 
 cudaError_t launch_frame_first(const PipeParams& p, uint32_t threads, uint32_t opt, int smCount, cudaStream_t s,
@@ -902,7 +1132,7 @@ cudaError_t launch_frame_late(const PipeParams& p, int smCount, cudaStream_t s, 
     q.descending = 0u;
     cudaError_t e = launch_pdl(frame_late_kernel<kFrameLateThreads>, grid, kFrameLateThreads, 0, s, q);
     if (e != cudaSuccess || !scatter) return e;
-    return launch_pdl(cull_scatter_kernel<true>, scatter_blocks(q), kScatterWarps * 32, 0, s, q);
+    return launch_pdl(cull_scatter_kernel, scatter_blocks(q), kScatterWarps * 32, 0, s, q);
 }
 
 cudaError_t launch_frame_scatter2(const PipeParams& p1, const PipeParams& p2, cudaStream_t s) {
@@ -912,13 +1142,17 @@ cudaError_t launch_frame_scatter2(const PipeParams& p1, const PipeParams& p2, cu
     return launch_pdl(cull_scatter2_kernel, g1 + g2, kScatterWarps * 32, 0, s, q1, q2, g1);
 }
 
+// Pass 1's blocks hold a candidate queue beside the survivor ring, which 16 warps do not fit in 48 KB
+// of static shared memory: the 512 x 1 shape runs as twice the blocks of 256 x 1.
+__host__ constexpr uint32_t first_threads(uint32_t threads) { return threads == 512u ? 256u : threads; }
+
 template <int MODE>
 static uint32_t single_blocks_per_sm(uint32_t threads, uint32_t opt) {
     if (threads == 256 && opt == 1) return occupancy_t<MODE, true, 256, 1>();
     if (threads == 256 && opt == 4) return occupancy_t<MODE, true, 256, 4>();
     if (threads == 128 && opt == 2) return occupancy_t<MODE, true, 128, 2>();
     if (threads == 128 && opt == 4) return occupancy_t<MODE, true, 128, 4>();
-    if (threads == 512 && opt == 1) return occupancy_t<MODE, true, 512, 1>();
+    if (threads == 512 && opt == 1) return occupancy_t<MODE, true, MODE == BLZ_MODE_FIRST ? first_threads(512) : 512, 1>();
     return occupancy_t<MODE, true, kObjThreads, kObjOpt>();
 }
 
@@ -937,6 +1171,7 @@ uint32_t single_chunk_size(uint32_t mode, uint32_t threads, uint32_t opt, uint32
         case kModeInstanced: per = single_blocks_per_sm<kModeInstanced>(threads, opt); break;
         default: per = single_blocks_per_sm<BLZ_MODE_FRUSTUM>(threads, opt); break;
     }
+    if (mode == BLZ_MODE_FIRST) threads = first_threads(threads);
     const uint64_t warps = static_cast<uint64_t>(per) * static_cast<uint64_t>(smCount > 0 ? smCount : 1) * (threads / 32u);
     const uint32_t step = 32u * opt;
     uint64_t size = (count + warps - 1) / warps;
@@ -955,7 +1190,7 @@ static cudaError_t launch_single_mode(const PipeParams& p, uint32_t threads, uin
     if (threads == 256 && opt == 4) return launch_t<MODE, true, 256, 4>(p, 0, smCount, s);
     if (threads == 128 && opt == 2) return launch_t<MODE, true, 128, 2>(p, 0, smCount, s);
     if (threads == 128 && opt == 4) return launch_t<MODE, true, 128, 4>(p, 0, smCount, s);
-    if (threads == 512 && opt == 1) return launch_t<MODE, true, 512, 1>(p, 0, smCount, s);
+    if (threads == 512 && opt == 1) return launch_t<MODE, true, MODE == BLZ_MODE_FIRST ? first_threads(512) : 512, 1>(p, 0, smCount, s);
     return launch_t<MODE, true, kObjThreads, kObjOpt>(p, 0, smCount, s);
 }
 
@@ -1304,7 +1539,11 @@ bool batch_shape_supported(uint32_t threads, uint32_t opt) {
 }
 
 // A batch whose views all run one pass takes a kernel compiled for that pass: without the other
-// passes' code it fits 64 registers, twice the resident warps of the per-view-mode kernel (112).
+// passes' code it fits 64 registers, twice the resident warps of the per-view-mode kernel. The default
+// shape's two objects per thread do not (79 registers, or spills: 213 and 237 us for the 64-view batch
+// against 202), so it runs as 256 x 1 too. That batch took 303 us with the per-view-mode kernel, every view
+// reading the 128 MB table from memory for itself; its floor is 45 us of memory traffic, and what is left
+// is 185 instructions per 32 objects at half the issue rate.
 template <int MODE>
 static cudaError_t launch_batch_mode(const PipeParams& p, uint32_t threads, uint32_t blocksPerSm, int smCount,
                                      cudaStream_t s) {
@@ -1314,7 +1553,7 @@ static cudaError_t launch_batch_mode(const PipeParams& p, uint32_t threads, uint
 
 cudaError_t launch_batch_cull(const PipeParams& p, uint32_t threads, uint32_t opt, uint32_t blocksPerSm, int smCount,
                               cudaStream_t s, int mode) {
-    if (mode >= 0 && opt == 1 && (threads == 256 || threads == 512)) {
+    if (mode >= 0 && (threads == 256 ? opt <= 2 : threads == 512 && opt == 1)) {
         switch (mode) {
             case BLZ_MODE_FRUSTUM: return launch_batch_mode<BLZ_MODE_FRUSTUM>(p, threads, blocksPerSm, smCount, s);
             case BLZ_MODE_FIRST: return launch_batch_mode<BLZ_MODE_FIRST>(p, threads, blocksPerSm, smCount, s);

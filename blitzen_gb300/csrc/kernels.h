@@ -110,6 +110,8 @@ struct PipeParams {
     Scratch* scratch;      // status word
     uint2* staged;         // [totalTiles * chunkSize] (objectId, lodId)
     uint32_t* chunkCount;  // [totalTiles]
+    uint2* chunkBase;      // batches: [totalTiles] {offset of the chunk's records in its view's, view}
+    const uint32_t* order; // batches: the chunks in the order they are decided, or NULL: by index
     unsigned int* workCounter;  // next chunk to decide (zero between launches), or NULL: static chunks
     void* keep;            // kept frame: [totalTiles * chunkSize] survivors (32 bytes each) pass 1 keeps for pass 2
     uint32_t* keepCount;   // kept frame: [totalTiles] survivors per chunk
@@ -227,6 +229,13 @@ inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, 
 }
 
 uint32_t object_tile_size();
+// The decide order of a batch whose views read a transform table that does not stay in L2 (see
+// batch_order_kernel; p: tileStart, viewCount, totalTiles; largest: the most chunks a view has). Worth its 3 us from tables of kBatchOrderBytes
+// on; up to kBatchOrderViews views.
+constexpr uint32_t kBatchOrderViews = 256;
+constexpr size_t kBatchOrderBytes = size_t(48) << 20;
+constexpr uint32_t kBatchOrderChunks = 4096;
+cudaError_t launch_batch_order(const PipeParams& p, uint32_t largest, uint32_t* order, cudaStream_t s);
 // Chunk size of a single-view launch of `count` objects: one chunk per warp the launch holds
 // resident, so every warp streams one contiguous run of objects and none waits for a second round.
 // (Smaller chunks handed out by a counter measured slower: each chunk drains its survivor ring in

@@ -398,7 +398,7 @@ int blz_batch_graph_destroy(blz_batch_graph* g);
  * 256, 512 or 1024, 0 = 512). blz_set_launch_shape also sets the single-view kernels' threads and
  * objects per thread when they have that shape (256 x 1, 2 or 4; 128 x 2 or 4; 512 x 1), and
  * forgets every choice the autotuners cached. A batch whose views all run the same pass uses a
- * kernel compiled for that pass for 256 x 1 and 512 x 1.
+ * kernel compiled for that pass for 256 x 1 (as which 256 x 2 runs too) and 512 x 1.
  *
  * blz_autotune_batch times every batch shape (threads x objects per thread x blocks per SM x chunk
  * size) on the given batch, keeps the fastest as the context's shape and caches it for the batch's
