@@ -643,9 +643,10 @@ static int object_cull(blz_ctx* c, uint32_t mode, const BlzCameraViewData* view,
     p.chunkSize = tile;
     bind_chunk_scratch(c, p);
     p.workCounter = nullptr;  // one chunk per resident warp, assigned by warp index
-    cudaError_t e = launch_object_cull(mode, p, threads, opt, c->smCount, reinterpret_cast<cudaStream_t>(stream));
+    uint32_t launches = 0;
+    cudaError_t e = launch_object_cull(mode, p, threads, opt, c->smCount, reinterpret_cast<cudaStream_t>(stream), &launches);
     if (e != cudaSuccess) return cuda_fail(e, "cull launch");
-    c->launches += 2;  // decide + scatter
+    c->launches += launches;
     return BLZ_OK;
 }
 

@@ -532,10 +532,13 @@ struct DecideSmem {
 };
 
 // The decide kernels' body: each warp decides chunks of a view (decide_run_warp) and records each
-// chunk's count. kModeFramePyr passes the context's pyramid-ready flag and its wait limit.
-template <int MODE, bool SINGLE, int THREADS, int OPT>
-__device__ __forceinline__ void decide_body(const PipeParams& p, DecideSmem<MODE, SINGLE, THREADS, OPT>& sm,
-                                            const unsigned int* ready = nullptr, uint32_t spinLimit = 0u) {
+// chunk's count; the count of the warp's last chunk is returned (0 when it had none). kModeFramePyr
+// passes the context's pyramid-ready flag and its wait limit. LOCAL: one chunk a warp at most, its
+// records staged at warpStage and its count only returned.
+template <int MODE, bool SINGLE, int THREADS, int OPT, bool LOCAL = false>
+__device__ __forceinline__ uint32_t decide_body(const PipeParams& p, DecideSmem<MODE, SINGLE, THREADS, OPT>& sm,
+                                                const unsigned int* ready = nullptr, uint32_t spinLimit = 0u,
+                                                uint2* warpStage = nullptr) {
     using Smem = DecideSmem<MODE, SINGLE, THREADS, OPT>;
     constexpr int NW = Smem::NW;
     constexpr uint32_t kSurf = Smem::kSurf;
@@ -561,6 +564,7 @@ __device__ __forceinline__ void decide_body(const PipeParams& p, DecideSmem<MODE
     const uint32_t warpsTotal = gridDim.x * NW;
     const uint32_t chunkSize = p.chunkSize;
     unsigned int flags = 0u;
+    uint32_t last = 0u;
     // every warp starts on the chunk of its index; later chunks come from the work counter when
     // there is one (a warp that finishes early takes the next, so warps finish together), else by
     // a stride of the grid's warp count
@@ -582,7 +586,7 @@ __device__ __forceinline__ void decide_body(const PipeParams& p, DecideSmem<MODE
         const BatchViewDev& bv = view_of<SINGLE>(p, vi);
         const uint32_t base = (chunk - first) * chunkSize;
         const uint32_t limit = min(base + chunkSize, bv.count);
-        uint2* stage = p.staged + static_cast<size_t>(chunk) * chunkSize;
+        uint2* stage = LOCAL ? warpStage : p.staged + static_cast<size_t>(chunk) * chunkSize;
         auto& ring = sm.ring[warp];
         auto& cand = sm.cand[warp];
         SharedView* shared = &sm.view[SINGLE ? 0u : warp];
@@ -604,14 +608,16 @@ __device__ __forceinline__ void decide_body(const PipeParams& p, DecideSmem<MODE
             total = decide_run_warp<(MODE < 0 ? 0 : MODE), SINGLE, OPT>(p.sc, bv, base, limit, stage, ring, cand, surf, shared, flags, keep, kept,
                                                                        stage1, &total1, ready, spinLimit, hist);
         }
-        if (lane == 0) {
+        if (!LOCAL && lane == 0) {
             p.chunkCount[chunk] = total;
             if constexpr (MODE == kModeFrame1) p.keepCount[chunk] = kept;
             if constexpr (fused_mode(MODE)) p.chunkCount2[chunk] = total1;
         }
+        last = total;
         item = next;
     }
     if (flags) atomicOr(&p.scratch->status, flags);
+    return last;
 }
 
 template <int MODE, bool SINGLE, int THREADS, int OPT>
@@ -755,6 +761,71 @@ __device__ __forceinline__ void scatter_block(const PipeParams& p, const uint32_
 __global__ void __launch_bounds__(kScatterWarps * 32, 2) cull_scatter_kernel(const PipeParams p) {
     pdl_wait();
     scatter_block(p, blockIdx.x);
+}
+
+// A short list in one launch: up to kSmallChunks chunks, one per warp of one cluster. The decide body stages
+// the chunk's records in shared memory; the warp hands its count to every block of the cluster (distributed
+// shared memory) and, behind the cluster's barrier, knows where its records go and writes them, the draw
+// count with them. While the barrier completes it fetches its records' LODs. Bound by that chain of latencies:
+// of two launches the second costs a dependent start, a reload of the counts and two block barriers. Replayed
+// back to back, 1,000 to 4,096 objects take 3.7 to 4.4 us a call by the pass; two launches took 4.75 to 5.4 (4,097
+// objects take that still). Lists of more than a step per warp stay with two launches: a further step costs
+// about what the second launch does.
+constexpr uint32_t kSmallBlocks = 8;  // the portable cluster size
+constexpr uint32_t kSmallChunks = kSmallBlocks * (kObjThreads / 32);
+constexpr uint32_t kSmallChunkSize = 32 * kObjOpt;
+
+template <int MODE>
+__global__ void __launch_bounds__(kObjThreads) cull_small_kernel(const PipeParams p) {
+    constexpr uint32_t NW = kObjThreads / 32;
+    __shared__ DecideSmem<MODE, true, kObjThreads, kObjOpt> sm;
+    __shared__ uint32_t s_count[kSmallChunks];
+    __shared__ uint2 s_stage[NW][kSmallChunkSize];
+    // every block of the cluster is running before the first write to its shared memory (awaited below)
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    pdl_wait();
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, chunk = blockIdx.x * NW + warp;
+    const uint32_t n = decide_body<MODE, true, kObjThreads, kObjOpt, true>(p, sm, nullptr, 0u, s_stage[warp]);
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    if (lane < gridDim.x) {  // one cluster is the whole grid: lane k writes block k's copy
+        const uint32_t mine = static_cast<uint32_t>(__cvta_generic_to_shared(&s_count[chunk]));
+        uint32_t theirs;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(theirs) : "r"(mine), "r"(lane));
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(theirs), "r"(n) : "memory");
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    uint2 rec[kObjOpt], lod[kObjOpt];
+#pragma unroll
+    for (uint32_t u = 0; u < kObjOpt; ++u) {
+        const uint32_t i = lane + 32u * u;
+        rec[u] = i < n ? s_stage[warp][i] : make_uint2(0u, 0u);
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < kObjOpt; ++u)
+        lod[u] = lane + 32u * u < n ? ldp(reinterpret_cast<const uint2*>(p.sc.lods + rec[u].y)) : make_uint2(0u, 0u);
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    uint32_t base = 0, total = 0;
+    for (uint32_t c = lane; c < gridDim.x * NW; c += 32u) {
+        const uint32_t x = s_count[c];
+        total += x;
+        if (c < chunk) base += x;
+    }
+    base = __reduce_add_sync(0xFFFFFFFFu, base);
+    const BatchViewDev& bv = p.single;
+    // staged record i goes to slot base + i, or base + n - 1 - i for a chunk staged last object first
+#pragma unroll
+    for (uint32_t u = 0; u < kObjOpt; ++u) {
+        const uint32_t i = lane + 32u * u, slot = base + (MODE == BLZ_MODE_LATE ? n - 1u - i : i);
+        if (i < n && slot < bv.capacity) put_record(bv.cmds, bv.stride, slot, rec[u].x, lod[u].x, lod[u].y);
+    }
+    if (chunk == 0u) {
+        total = __reduce_add_sync(0xFFFFFFFFu, total);
+        if (lane == 0u) {
+            *bv.drawCount = total;
+            if (total > bv.capacity) atomicOr(&p.scratch->status, BLZ_FLAG_COMMAND_OVERFLOW);
+        }
+    }
 }
 
 // Batched views: two launches. The scan has a block per view: it scans the counts of the view's chunks into
@@ -1184,8 +1255,34 @@ bool single_shape_supported(uint32_t threads, uint32_t opt) {
            (threads == 512 && opt == 1);
 }
 
+// One launch for the default shape's short lists, where every warp has one step of one chunk and all warps
+// fit one cluster: up to 4,096 objects (measured on both sides of the line: cull_small_kernel).
+static bool small_list(const PipeParams& p, uint32_t threads, uint32_t opt) {
+    return (threads == kObjThreads && opt == kObjOpt) && p.totalTiles <= kSmallChunks && p.chunkSize == kSmallChunkSize;
+}
+
+template <int MODE>
+static cudaError_t launch_small_t(const PipeParams& p, cudaStream_t s) {
+    constexpr uint32_t NW = kObjThreads / 32;
+    uint32_t blocks = 1;
+    while (blocks * NW < p.totalTiles) blocks *= 2u;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = blocks;
+    cfg.blockDim = kObjThreads;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim = {blocks, 1, 1};
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, cull_small_kernel<MODE>, p);
+}
+
 template <int MODE>
 static cudaError_t launch_single_mode(const PipeParams& p, uint32_t threads, uint32_t opt, int smCount, cudaStream_t s) {
+    if (small_list(p, threads, opt)) return launch_small_t<MODE>(p, s);
     if (threads == 256 && opt == 1) return launch_t<MODE, true, 256, 1>(p, 0, smCount, s);
     if (threads == 256 && opt == 4) return launch_t<MODE, true, 256, 4>(p, 0, smCount, s);
     if (threads == 128 && opt == 2) return launch_t<MODE, true, 128, 2>(p, 0, smCount, s);
@@ -1195,7 +1292,8 @@ static cudaError_t launch_single_mode(const PipeParams& p, uint32_t threads, uin
 }
 
 cudaError_t launch_object_cull(uint32_t mode, const PipeParams& p, uint32_t threads, uint32_t opt, int smCount,
-                               cudaStream_t s) {
+                               cudaStream_t s, uint32_t* launches) {
+    *launches = small_list(p, threads, opt) ? 1u : 2u;  // decide + scatter
     PipeParams q = p;
     q.descending = mode == BLZ_MODE_LATE ? 1u : 0u;  // the single-view pass-2 decide walks its chunks downwards
     switch (mode) {

@@ -243,7 +243,7 @@ cudaError_t launch_batch_order(const PipeParams& p, uint32_t largest, uint32_t* 
 uint32_t single_chunk_size(uint32_t mode, uint32_t threads, uint32_t opt, uint32_t count, int smCount);
 bool single_shape_supported(uint32_t threads, uint32_t opt);
 cudaError_t launch_object_cull(uint32_t mode, const PipeParams& p, uint32_t threads, uint32_t opt, int smCount,
-                               cudaStream_t s);
+                               cudaStream_t s, uint32_t* launches);
 // A kept frame (blz_frame_first / blz_frame_late): pass 1 tests every object once and keeps the
 // frustum survivors in p.keep; pass 2 runs the pyramid test over those alone. `scatter` false leaves
 // the records staged.

@@ -102,9 +102,10 @@ extern "C" int blz_cull_frustum_noalloc(blz_ctx* c, const BlzCameraViewData* vie
     p.scratch = c->scratch;  // status flags stay in the context, read by blz_ctx_check
     p.staged = reinterpret_cast<uint2*>(base);
     p.chunkCount = reinterpret_cast<uint32_t*>(base + kCountsOffset);
+    uint32_t launches = 0;
     e = launch_object_cull(BLZ_MODE_FRUSTUM, p, c->singleThreads, c->singleOpt, c->smCount,
-                           reinterpret_cast<cudaStream_t>(stream));
+                           reinterpret_cast<cudaStream_t>(stream), &launches);
     if (e != cudaSuccess) return cuda_fail(e, "no-alloc cull launch");
-    c->launches += 2;  // decide + scatter
+    c->launches += launches;
     return BLZ_OK;
 }
