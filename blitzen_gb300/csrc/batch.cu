@@ -283,6 +283,7 @@ int blz_cull_batch_per_view(blz_ctx* c, const BlzBatchView* views, uint32_t n, b
         p.totalTiles = ts[i + 1] - ts[i];
         p.chunkSize = tile;
         bind_chunk_scratch(c, p);
+        p.workCounter = nullptr;  // chunks by a stride: only a batch's scan rewinds the counter
         uint32_t launches = 0;
         cudaError_t e = launch_object_cull(d[i].mode, p, c->singleThreads, c->singleOpt, c->smCount, st, &launches);
         if (e != cudaSuccess) return cuda_fail(e, "per-view cull launch");
