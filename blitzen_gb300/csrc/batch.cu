@@ -20,6 +20,17 @@ static uint32_t batch_chunk(const BlzLaunchShape& s) { return s.chunkObjects ? s
 
 static bool chunk_supported(uint32_t chunk) { return chunk == 0 || chunk == 256 || chunk == 512 || chunk == 1024; }
 
+// Chunk of a batch of `objects` in all. A chunk is one warp's work, and a warp's time its steps one after another,
+// so a batch too small to give every resident warp of the default shape (kBatchWarpsPerSm an SM) a chunk of 512
+// is cut finer, down to one step. Shapes that name their chunk keep it.
+static uint32_t batch_chunk_for(const BlzLaunchShape& s, uint64_t objects, int smCount) {
+    uint32_t chunk = batch_chunk(s);
+    if (s.chunkObjects || s.threadsPerBlock != kObjThreads || s.objectsPerThread != kObjOpt) return chunk;
+    const uint64_t warps = static_cast<uint64_t>(smCount > 0 ? smCount : 1) * kBatchWarpsPerSm;
+    while (chunk > 32u * kObjOpt && objects <= warps * (chunk / 2u)) chunk /= 2u;
+    return chunk;
+}
+
 const TunedShape* find_tuned(const blz_ctx* c, uint64_t objects, uint32_t views, uint32_t mode) {
     for (const TunedShape& t : c->tuned)
         if (t.objects == objects && t.views == views && t.mode == mode) return &t;
@@ -146,7 +157,7 @@ static int uniform_mode(const BlzBatchView* views, uint32_t n) {
 // Whether the chunks are decided in the order of batch_order_kernel: several views, enough chunks for it to
 // matter, and a transform table that would be read from memory again for each view.
 static bool wants_order(const PipeParams& p) {
-    return p.viewCount > 1 && p.viewCount <= kBatchOrderViews && p.totalTiles >= kBatchOrderChunks &&
+    return p.viewCount > 1 && p.viewCount <= kBatchOrderViews && static_cast<uint64_t>(p.totalTiles) * p.chunkSize >= kBatchOrderObjects &&
            p.sc.transformCount * sizeof(BlzMeshTransform) >= kBatchOrderBytes;
 }
 
@@ -157,7 +168,7 @@ static uint32_t largest_view(const std::vector<uint32_t>& tileStart) {
 }
 
 static int run_batch_shape(blz_ctx* c, const BlzBatchView* views, uint32_t n, cudaStream_t st, const BlzLaunchShape& sh) {
-    const uint32_t tile = batch_chunk(sh);
+    const uint32_t tile = batch_chunk_for(sh, batch_objects(c, views, n), c->smCount);
     std::vector<BatchViewDev> d;
     std::vector<uint32_t> ts;
     int rc = build_views(c, views, n, tile, d, ts);
@@ -372,7 +383,7 @@ int blz_batch_graph_create(blz_ctx* c, const BlzBatchView* views, uint32_t n, bl
     *outGraph = nullptr;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const BlzLaunchShape sh = batch_shape(c, views, n);
-    const uint32_t tile = batch_chunk(sh);
+    const uint32_t tile = batch_chunk_for(sh, batch_objects(c, views, n), c->smCount);
     std::vector<BatchViewDev> d;
     std::vector<uint32_t> ts;
     int rc = build_views(c, views, n, tile, d, ts);

@@ -234,7 +234,12 @@ uint32_t object_tile_size();
 // on; up to kBatchOrderViews views.
 constexpr uint32_t kBatchOrderViews = 256;
 constexpr size_t kBatchOrderBytes = size_t(48) << 20;
-constexpr uint32_t kBatchOrderChunks = 4096;
+constexpr uint64_t kBatchOrderObjects = uint64_t(1) << 21;
+// Warps an SM for which a batch of the default shape is cut into chunks. Whole calls of 30 views of 0.4M objects in
+// all, 2 of 9k and 16 of 0.5M took 34, 30 and 50 us with chunks of 512; cut for 16 warps an SM 27.5, 18 and 34, for
+// 32 23, 18 to 20 and 31, for 64 23, 18 and 31. At 2M objects (32 views) 32 keeps chunks of 512; 64 gained 6% on one
+// pass and lost nothing, but doubles the scratch slots.
+constexpr uint32_t kBatchWarpsPerSm = 32;
 cudaError_t launch_batch_order(const PipeParams& p, uint32_t largest, uint32_t* order, cudaStream_t s);
 // Chunk size of a single-view launch of `count` objects: one chunk per warp the launch holds
 // resident, so every warp streams one contiguous run of objects and none waits for a second round.

@@ -205,8 +205,8 @@ typedef struct BlzPyramid {
 uint64_t blz_pyramid_layout(uint32_t depthWidth, uint32_t depthHeight, uint32_t mode, BlzPyramid* out);
 
 /* Builds every mip from an fp32 reverse-Z depth buffer (row-major, depthWidth floats per row):
- * one launch for the 32x32 tiles and one for the top mips. Replaces GenerateDepthPyramid
- * (src/Renderer/BlitzenDX12/dx12Draw.cpp:224-288, src/Renderer/BlitzenVulkan/vulkanDraw.cpp:554-622)
+ * one launch: a block per 32x32 tile, the block that finishes last building the top mips. Replaces
+ * GenerateDepthPyramid (src/Renderer/BlitzenDX12/dx12Draw.cpp:224-288, src/Renderer/BlitzenVulkan/vulkanDraw.cpp:554-622)
  * and its per-mip dispatches of depthPyramid.cs.hlsl / DepthPyramidGeneration.comp.glsl.
  * dDepth is any device-accessible pointer: device memory, or pinned host memory that the kernel
  * then reads once over the CPU-GPU link (no separate upload). */
@@ -395,7 +395,8 @@ int blz_batch_graph_destroy(blz_batch_graph* g);
 
 /* Launch shape used by the batch kernel: threads per block, objects per thread, blocks per SM and
  * objects per chunk (the compaction unit: each chunk's records are staged and counted together;
- * 256, 512 or 1024, 0 = 512). blz_set_launch_shape also sets the single-view kernels' threads and
+ * 256, 512 or 1024; 0 = 512, cut down to 64 for a batch of 256 x 2 too small to give each resident
+ * warp a chunk of 512). blz_set_launch_shape also sets the single-view kernels' threads and
  * objects per thread when they have that shape (256 x 1, 2 or 4; 128 x 2 or 4; 512 x 1), and
  * forgets every choice the autotuners cached. A batch whose views all run the same pass uses a
  * kernel compiled for that pass for 256 x 1 (as which 256 x 2 runs too) and 512 x 1.
