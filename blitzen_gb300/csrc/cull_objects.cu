@@ -1,10 +1,11 @@
 // cull_objects.cu — per-object cull kernels: frustum, occlusion pass 1 / pass 2, temporal
 // occlusion, for one view or many views in one launch.
 //
-// Two or three kernels per launch, no block ever waiting on another:
+// Two or three kernels per call, no block ever waiting on another (lists of up to 4,096 objects: one kernel
+// doing both steps, its blocks meeting at their cluster's barrier, cull_small_kernel):
 //   decide   a streaming grid of warps, each deciding contiguous chunks of a view's render objects
-//            (single views: one chunk per resident warp, assigned by warp index; batches: 512-object
-//            chunks of all views, taken from a work counter), staging the emitted ones compacted in
+//            (single views: one chunk per resident warp, assigned by warp index; batches: chunks
+//            of 64 to 1024 objects of all views, taken from a work counter), staging the emitted ones compacted in
 //            object order — (objectId, lodId), 8 bytes — in the chunk's slice of a scratch buffer,
 //            with the chunk's count;
 //   scatter  finds the chunks' output offsets from the counts, copies the staged records to their final
@@ -58,7 +59,7 @@ __device__ __forceinline__ uint32_t find_view_warp(const uint32_t* tileStart, ui
 
 // ------------------------------------------------------------------ decisions
 
-constexpr uint32_t kChunk = 512;  // objects per chunk of batched views (single views size theirs)
+constexpr uint32_t kChunk = 512;  // objects per chunk of batched views, unless the shape or a small batch wants others (single views size theirs)
 // Chunks per group of the instanced counting sort. 16 and 8 took 46.0 and 48.7 us against 44.9 for the
 // instanced pass of 4M objects and 256 LODs, 24.5 and 31.3 against 18.6 for 250k and 2000 (more rows to
 // scan, fewer warps to place them).
