@@ -782,20 +782,22 @@ __global__ void __launch_bounds__(kObjThreads) cull_small_kernel(const PipeParam
     __shared__ DecideSmem<MODE, true, kObjThreads, kObjOpt> sm;
     __shared__ uint32_t s_count[kSmallChunks];
     __shared__ uint2 s_stage[NW][kSmallChunkSize];
-    // every block of the cluster is running before the first write to its shared memory (awaited below)
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    // Every block of the cluster is running before the first write to its shared memory (awaited below). The
+    // barriers are not of the .aligned form: the second arrive follows a branch that some lanes do not take,
+    // and that form wants the warp's lanes together, which nothing here promises.
+    asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
     pdl_wait();
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, chunk = blockIdx.x * NW + warp;
     const uint32_t n = decide_body<MODE, true, kObjThreads, kObjOpt, true>(p, sm, nullptr, 0u, s_stage[warp]);
     __syncwarp();
-    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait;" ::: "memory");
     if (lane < gridDim.x) {  // one cluster is the whole grid: lane k writes block k's copy
         const uint32_t mine = static_cast<uint32_t>(__cvta_generic_to_shared(&s_count[chunk]));
         uint32_t theirs;
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(theirs) : "r"(mine), "r"(lane));
         asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(theirs), "r"(n) : "memory");
     }
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     uint2 rec[kObjOpt], lod[kObjOpt];
 #pragma unroll
     for (uint32_t u = 0; u < kObjOpt; ++u) {
@@ -805,7 +807,7 @@ __global__ void __launch_bounds__(kObjThreads) cull_small_kernel(const PipeParam
 #pragma unroll
     for (uint32_t u = 0; u < kObjOpt; ++u)
         lod[u] = lane + 32u * u < n ? ldp(reinterpret_cast<const uint2*>(p.sc.lods + rec[u].y)) : make_uint2(0u, 0u);
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
     uint32_t base = 0, total = 0;
     for (uint32_t c = lane; c < gridDim.x * NW; c += 32u) {
         const uint32_t x = s_count[c];
