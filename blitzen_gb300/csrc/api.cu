@@ -96,7 +96,12 @@ int ensure_chunk_scratch(blz_ctx* c, size_t chunks, size_t chunkSize) {
     if (objects <= c->chunkObjects && chunks <= c->chunkSlots) return BLZ_OK;
     if (c->capturing) return fail(BLZ_ERR_CAPACITY, "scratch must grow, which a capture cannot record: run the calls once before capturing");
     size_t wantObj = objects > c->chunkObjects ? objects + objects / 4 : c->chunkObjects;
+    // A graph recorded on this context holds this block's address, so the block may not move for a call whose
+    // records it has room for: it has a slot for every 64 of its objects, the finest chunk a batch is cut into,
+    // and only a call of more objects grows it. (A list of 321,000 objects is decided in 2,508 chunks of 128,
+    // a batch of 300,000 in 4,700 chunks of 64.)
     size_t wantSlots = chunks > c->chunkSlots ? chunks + chunks / 4 + 64 : c->chunkSlots;
+    wantSlots = std::max(wantSlots, wantObj / 64 + 64);
     if (c->chunkMem) {
         cudaDeviceSynchronize();
         cudaFree(c->chunkMem);
