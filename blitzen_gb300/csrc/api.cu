@@ -310,6 +310,7 @@ int blz_ctx_debug_advance_ticket(blz_ctx* c, uint32_t n, blz_stream_t stream) {
     if (n == 0 || n > 1024) return fail(BLZ_ERR_INVALID_ARGUMENT, "ticket advance %u outside [1, 1024]", n);
     cudaError_t e = launch_add_word(&c->scratch->ticket, n, reinterpret_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(e, "ticket advance");
+    c->ticketAdvanced = true;
     return BLZ_OK;
 }
 
@@ -1005,16 +1006,17 @@ int blz_cull_instanced(blz_ctx* c, const BlzCameraViewData* view, BlzRenderList 
     // Scenes of many LODs also have a form that needs no scratch, one launch in which tiles wait for one
     // another: 38 us against 15 for 250k objects and 2000 LODs, but a recorded call keeps it, since it
     // needs no earlier call to have sized anything and stays valid whatever grows later, and so does a call
-    // whose scratch the device has no room for.
+    // whose scratch the device has no room for, and the one after the test hook that advances its ticket.
     const size_t words = static_cast<size_t>(groups + 1u) * nL;  // the groups' histograms, then the LODs' totals
     const size_t staged = static_cast<size_t>(chunks) * tile;
-    bool sorted = true;
+    bool sorted = true, recorded = false;
     if (!manyLods) {
         rc = ensure_chunk_scratch(c, chunks, tile);
         if (rc == BLZ_OK) rc = ensure_instanced_words(c, words);
         if (rc != BLZ_OK) return rc;
     } else {
-        sorted = !stream_capturing(reinterpret_cast<cudaStream_t>(s)) &&
+        recorded = stream_capturing(reinterpret_cast<cudaStream_t>(s));
+        sorted = !recorded && !c->ticketAdvanced &&
                  ensure_many_lods_scratch(c, staged * sizeof(uint2) + (chunks + words) * sizeof(uint32_t)) == BLZ_OK;
     }
     if (sorted) {
@@ -1054,10 +1056,6 @@ int blz_cull_instanced(blz_ctx* c, const BlzCameraViewData* view, BlzRenderList 
         q.capacity = target->capacity;
         q.drawCount = target->drawCount;
         q.status = &c->scratch->status;
-        if (manyLods) {
-            q.ticket = &c->scratch->ticket;
-            q.ticketDone = &c->scratch->doneBlocks;
-        }
         cudaError_t e = launch_instanced_staged(p, q, c->singleThreads, c->singleOpt, c->smCount, reinterpret_cast<cudaStream_t>(s));
         if (e != cudaSuccess) return cuda_fail(e, "instanced cull launch");
         c->launches += 4;  // the group histograms' zeroing, decide, scan, place
@@ -1079,6 +1077,7 @@ int blz_cull_instanced(blz_ctx* c, const BlzCameraViewData* view, BlzRenderList 
     p.spinLimit = c->waitLimit;
     cudaError_t e = launch_instanced_cull(p, *view, reinterpret_cast<cudaStream_t>(s));
     if (e != cudaSuccess) return cuda_fail(e, "instanced cull launch");
+    if (!recorded) c->ticketAdvanced = false;  // the launch rewinds the ticket
     c->launches++;
     return BLZ_OK;
 }

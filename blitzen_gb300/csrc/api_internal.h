@@ -49,6 +49,7 @@ struct blz_ctx {
     size_t instWords = 0;
     void* manyLodsMem = nullptr;       // instanced cull above kInstStagedMaxLods LODs: staged records, chunk counts, histograms, totals
     size_t manyLodsBytes = 0;
+    bool ticketAdvanced = false;       // test hook: the next direct instanced cull of many LODs takes the form that waits
     void* clusterMem = nullptr;        // cluster cull: tile counts, object ranges and survivors, visibility bits
     size_t clusterBytes = 0;
     int clusterTestBlocksPerSm[2] = {0, 0};  // records, task form: resident test blocks per SM (found on first use)

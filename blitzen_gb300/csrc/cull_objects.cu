@@ -1391,30 +1391,24 @@ __global__ void __launch_bounds__(kInstGroup * 32) inst_place_kernel(const InstS
     extern __shared__ __align__(16) uint32_t s_rows[];
     __shared__ unsigned int s_flags;
     __shared__ uint32_t s_warpSums[32];
-    __shared__ uint32_t s_group;
     pdl_wait();
     const uint32_t T = blockDim.x, W = T / 32u, per = kInstGroup / W;
-    const uint32_t nL = q.nL, nS = inst_stride(nL), G = q.groups;
+    const uint32_t nL = q.nL, nS = inst_stride(nL), G = q.groups, g = blockIdx.x;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     uint32_t* s_goff = s_rows + W * nS;
     uint32_t* s_ioff = s_goff + nS;
     uint32_t* s_part = s_ioff + nS;
-    if (threadIdx.x == 0) {
-        s_flags = 0u;
-        s_group = q.ticket ? atomicAdd(q.ticket, 1u) : blockIdx.x;
-    }
+    if (threadIdx.x == 0) s_flags = 0u;
     for (uint32_t j = threadIdx.x; j < W * nS / 4u; j += T) reinterpret_cast<uint4*>(s_rows)[j] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
-    const uint32_t g = s_group;
-    const bool held = g < G;  // else a place past the grid: the tickets were left advanced
-    unsigned int flags = held ? 0u : BLZ_FLAG_TIMEOUT;
+    unsigned int flags = 0u;
     // the warp's records: those of its `per` chunks, one after another
     const uint32_t c0 = g * kInstGroup + warp * per;
     uint32_t first[kInstMaxPerWarp], n = 0;  // record index each chunk starts at
 #pragma unroll
     for (uint32_t k = 0; k < kInstMaxPerWarp; ++k) {
         first[k] = n;
-        if (held && k < per && c0 + k < q.totalTiles) n += __ldcg(q.chunkCount + c0 + k);
+        if (k < per && c0 + k < q.totalTiles) n += __ldcg(q.chunkCount + c0 + k);
     }
     auto record = [&](uint32_t j) -> uint2 {
         uint32_t k = 0, from = 0;
@@ -1434,7 +1428,7 @@ __global__ void __launch_bounds__(kInstGroup * 32) inst_place_kernel(const InstS
     load_batch(0, head);
     const uint32_t idBits = nL > 1u ? 32u - static_cast<uint32_t>(__clz(static_cast<int>(nL - 1u))) : 0u;
     for (uint32_t b = threadIdx.x; b < nL; b += T) {
-        s_goff[b] = held ? __ldcg(q.hist + static_cast<size_t>(g) * nL + b) : 0u;
+        s_goff[b] = __ldcg(q.hist + static_cast<size_t>(g) * nL + b);
         s_ioff[b] = __ldcg(&q.counters[b].instanceOffset);
     }
     uint32_t* row = s_rows + warp * nS;
@@ -1589,17 +1583,7 @@ __global__ void __launch_bounds__(kInstGroup * 32) inst_place_kernel(const InstS
     }
     if (flags) atomicOr(&s_flags, flags);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        if (s_flags) atomicOr(q.status, s_flags);
-        // the block that ends last rewinds the tickets
-        if (q.ticket) {
-            __threadfence();
-            if (atomicAdd(q.ticketDone, 1u) == G - 1u) {
-                *q.ticket = 0u;
-                *q.ticketDone = 0u;
-            }
-        }
-    }
+    if (threadIdx.x == 0 && s_flags) atomicOr(q.status, s_flags);
 }
 
 __global__ void __launch_bounds__(1024) zero_words_kernel(uint32_t* words, uint32_t n) {

@@ -157,8 +157,6 @@ struct InstStagedParams {
     uint32_t stride, capacity;
     uint32_t* drawCount;
     unsigned int* status;
-    unsigned int* ticket;       // groups are taken from this counter (zero between launches), or NULL: block g takes group g
-    unsigned int* ticketDone;   // blocks that have ended (zero between launches)
 };
 
 struct ClusterParams {
@@ -266,8 +264,8 @@ bool batch_shape_supported(uint32_t threads, uint32_t opt);
 cudaError_t launch_batch_cull(const PipeParams& p, uint32_t threads, uint32_t opt, uint32_t blocksPerSm, int smCount,
                               cudaStream_t s, int mode);
 uint32_t instanced_tile_size();
-// Above this many LODs the instanced cull's place launch takes its groups by ticket, and a recorded call
-// runs as one launch without scratch (launch_instanced_cull).
+// Above this many LODs the instanced cull's scratch is a block of its own, and a recorded call runs as one
+// launch without scratch (launch_instanced_cull).
 constexpr uint32_t kInstStagedMaxLods = 1024;
 uint32_t instanced_group_count(uint32_t chunks);
 cudaError_t launch_instanced_staged(const PipeParams& p, const InstStagedParams& q, uint32_t threads, uint32_t opt,

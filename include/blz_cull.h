@@ -92,8 +92,9 @@ const char* blz_version(void);
 int blz_ctx_check(blz_ctx* ctx, blz_stream_t stream, uint32_t* flagsOut);
 
 /* Bound of the device-side waits of this context's launches. Two kernels wait:
- *  - the instanced cull of scenes of more than 1,024 LODs when the call is recorded into a graph: a tile
- *    waits, per LOD, for the running totals of the tiles that started before it;
+ *  - the instanced cull of scenes of more than 1,024 LODs when the call is recorded into a graph, or the
+ *    device has no room for its scratch: a tile waits, per LOD, for the running totals of the tiles that
+ *    started before it;
  *  - the one-call frame given a depth buffer (blz_cull_frame): a warp waits, before its first Hi-Z
  *    test, for the pyramid the launch's blocks build first.
  * Each polls one word at most `polls` times; then it gives up, raises BLZ_FLAG_TIMEOUT and finishes
@@ -103,11 +104,11 @@ int blz_ctx_check(blz_ctx* ctx, blz_stream_t stream, uint32_t* flagsOut);
 int blz_ctx_set_wait_limit(blz_ctx* ctx, uint32_t polls);
 
 /* Test hook for the timeout path only: advances the context's block-ticket counter by n (1..1024)
- * on the stream, so that the next launch that takes tickets (the instanced cull of scenes of more than
- * 1,024 LODs) starts its blocks past the first n places. The blocks whose place lies past the launch's
- * end raise BLZ_FLAG_TIMEOUT, and in a recorded call, where blocks wait for places no block holds, those
- * waits run out first; the launch's last block rewinds the counter, so the launch after it is whole
- * again. No counterpart in the reference. */
+ * on the stream. The next launch that takes tickets, which is an instanced cull of more than 1,024
+ * LODs in its recorded form (a replay, or the next such call made directly: it takes that form too),
+ * starts its blocks past the first n places. Its blocks then wait for places no block holds, give up
+ * after the wait limit and raise BLZ_FLAG_TIMEOUT; the launch's last block rewinds the counter, so
+ * the launch after it is whole again. No counterpart in the reference. */
 int blz_ctx_debug_advance_ticket(blz_ctx* ctx, uint32_t n, blz_stream_t stream);
 
 /* Test hook for the one-call frame's wait only: advances the context's pyramid-tile ticket by n
