@@ -197,17 +197,25 @@ int cluster_test_occupancy(blz_ctx* c, bool tasks, ClusterParams& p) {
 }
 
 // Scratch of the instanced cull of scenes of many LODs, a block of its own: recorded calls never use it
-// (see blz_cull_instanced), so it can grow whatever has been recorded.
-static int ensure_many_lods_scratch(blz_ctx* c, size_t bytes) {
+// (see blz_cull_instanced), so it can grow whatever has been recorded. It can also grow while something is
+// being recorded elsewhere, by this thread or another: the allocation runs in relaxed capture mode, in which it
+// neither fails for that recording nor ends it, and waits for the call's own stream (a context serves one
+// stream at a time), not for the device.
+static int ensure_many_lods_scratch(blz_ctx* c, size_t bytes, cudaStream_t st) {
     if (bytes <= c->manyLodsBytes) return BLZ_OK;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
     if (c->manyLodsMem) {
-        cudaDeviceSynchronize();
+        cudaStreamSynchronize(st);
         cudaFree(c->manyLodsMem);
         c->manyLodsMem = nullptr;
         c->manyLodsBytes = 0;
     }
     const size_t want = bytes + bytes / 4;
-    if (cudaMalloc(&c->manyLodsMem, want) != cudaSuccess) {
+    const cudaError_t e = cudaMalloc(&c->manyLodsMem, want);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) {
+        c->manyLodsMem = nullptr;
         (void)cudaGetLastError();
         return fail(BLZ_ERR_OUT_OF_MEMORY, "instanced scratch of %zu bytes", want);
     }
@@ -268,7 +276,7 @@ int blz_ctx_create(int device, blz_ctx** out) {
         blz_ctx_destroy(c);
         return rc;
     }
-    if (ensure_many_lods_scratch(c, kFirstManyLodsBytes) != BLZ_OK) {
+    if (ensure_many_lods_scratch(c, kFirstManyLodsBytes, nullptr) != BLZ_OK) {
         blz_ctx_destroy(c);
         return fail(BLZ_ERR_OUT_OF_MEMORY, "scratch allocation failed");
     }
@@ -1017,7 +1025,7 @@ int blz_cull_instanced(blz_ctx* c, const BlzCameraViewData* view, BlzRenderList 
     } else {
         recorded = stream_capturing(reinterpret_cast<cudaStream_t>(s));
         sorted = !recorded && !c->ticketAdvanced &&
-                 ensure_many_lods_scratch(c, staged * sizeof(uint2) + (chunks + words) * sizeof(uint32_t)) == BLZ_OK;
+                 ensure_many_lods_scratch(c, staged * sizeof(uint2) + (chunks + words) * sizeof(uint32_t), reinterpret_cast<cudaStream_t>(s)) == BLZ_OK;
     }
     if (sorted) {
         PipeParams p{};
