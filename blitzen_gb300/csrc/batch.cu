@@ -53,9 +53,9 @@ static uint64_t batch_objects(const blz_ctx* c, const BlzBatchView* views, uint3
     return total;
 }
 
-// The shape a batch of these views runs with: the autotuner's choice for its size, else the context's.
-static BlzLaunchShape batch_shape(const blz_ctx* c, const BlzBatchView* views, uint32_t n) {
-    const TunedShape* t = find_tuned(c, batch_objects(c, views, n), n, kTunedBatch);
+// The shape a batch of n views runs with: the autotuner's choice for its size, else the context's.
+static BlzLaunchShape batch_shape(const blz_ctx* c, uint64_t objects, uint32_t n) {
+    const TunedShape* t = find_tuned(c, objects, n, kTunedBatch);
     return t ? t->shape : c->shape;
 }
 
@@ -106,6 +106,12 @@ static int build_views(blz_ctx* c, const BlzBatchView* views, uint32_t n, uint32
     return BLZ_OK;
 }
 
+static uint32_t largest_view(const std::vector<uint32_t>& tileStart) {
+    uint32_t most = 0;
+    for (size_t i = 1; i < tileStart.size(); ++i) most = std::max(most, tileStart[i] - tileStart[i - 1]);
+    return most;
+}
+
 static size_t batch_bytes(uint32_t n) { return sizeof(BatchViewDev) * n + sizeof(uint32_t) * (n + 1) + 256; }
 
 static int upload_views(blz_ctx* c, const std::vector<BatchViewDev>& d, const std::vector<uint32_t>& ts, void* dst,
@@ -128,6 +134,7 @@ static int upload_views(blz_ctx* c, const std::vector<BatchViewDev>& d, const st
     p.tileStart = reinterpret_cast<const uint32_t*>(static_cast<char*>(dst) + tsOff);
     p.viewCount = n;
     p.totalTiles = ts[n];
+    p.largest = largest_view(ts);
     p.chunkSize = tile;
     p.scratch = c->scratch;
     return BLZ_OK;
@@ -161,14 +168,8 @@ static bool wants_order(const PipeParams& p) {
            p.sc.transformCount * sizeof(BlzMeshTransform) >= kBatchOrderBytes;
 }
 
-static uint32_t largest_view(const std::vector<uint32_t>& tileStart) {
-    uint32_t most = 0;
-    for (size_t i = 1; i < tileStart.size(); ++i) most = std::max(most, tileStart[i] - tileStart[i - 1]);
-    return most;
-}
-
-static int run_batch_shape(blz_ctx* c, const BlzBatchView* views, uint32_t n, cudaStream_t st, const BlzLaunchShape& sh) {
-    const uint32_t tile = batch_chunk_for(sh, batch_objects(c, views, n), c->smCount);
+static int run_batch_shape(blz_ctx* c, const BlzBatchView* views, uint32_t n, uint64_t objects, cudaStream_t st, const BlzLaunchShape& sh) {
+    const uint32_t tile = batch_chunk_for(sh, objects, c->smCount);
     std::vector<BatchViewDev> d;
     std::vector<uint32_t> ts;
     int rc = build_views(c, views, n, tile, d, ts);
@@ -184,7 +185,7 @@ static int run_batch_shape(blz_ctx* c, const BlzBatchView* views, uint32_t n, cu
     cudaError_t e = cudaSuccess;
     if (wants_order(p)) {
         uint32_t* order = p.chunkCount + c->chunkSlots;
-        e = launch_batch_order(p, largest_view(ts), order, st);
+        e = launch_batch_order(p, order, st);
         p.order = order;
         c->launches++;
     }
@@ -198,7 +199,8 @@ static int run_batch_shape(blz_ctx* c, const BlzBatchView* views, uint32_t n, cu
 int run_batch(blz_ctx* c, const BlzBatchView* views, uint32_t n, cudaStream_t st) {
     if (!c || (n && !views)) return fail(BLZ_ERR_INVALID_ARGUMENT, "ctx or views is NULL");
     if (n == 0) return BLZ_OK;
-    return run_batch_shape(c, views, n, st, batch_shape(c, views, n));
+    const uint64_t objects = batch_objects(c, views, n);
+    return run_batch_shape(c, views, n, objects, st, batch_shape(c, objects, n));
 }
 
 }  // namespace blz
@@ -277,7 +279,7 @@ int blz_cull_batch_per_view(blz_ctx* c, const BlzBatchView* views, uint32_t n, b
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     std::vector<BatchViewDev> d;
     std::vector<uint32_t> ts;
-    const uint32_t tile = batch_chunk(batch_shape(c, views, n));
+    const uint32_t tile = batch_chunk(batch_shape(c, batch_objects(c, views, n), n));
     int rc = build_views(c, views, n, tile, d, ts);
     if (rc != BLZ_OK) return rc;
     uint32_t maxTiles = 1;
@@ -353,10 +355,10 @@ int blz_autotune_batch(blz_ctx* c, const BlzBatchView* views, uint32_t n, uint32
                     if (s && s * t > 2048) continue;
                     if (!batch_shape_supported(t, o)) continue;
                     const BlzLaunchShape sh{t, o, s, k};
-                    if (run_batch_shape(c, views, n, st, sh) != BLZ_OK) continue;  // warm-up
+                    if (run_batch_shape(c, views, n, objects, st, sh) != BLZ_OK) continue;  // warm-up
                     cudaEventRecord(a, st);
                     int rc = BLZ_OK;
-                    for (uint32_t r = 0; r < repeats && rc == BLZ_OK; ++r) rc = run_batch_shape(c, views, n, st, sh);
+                    for (uint32_t r = 0; r < repeats && rc == BLZ_OK; ++r) rc = run_batch_shape(c, views, n, objects, st, sh);
                     cudaEventRecord(b, st);
                     cudaEventSynchronize(b);
                     if (rc != BLZ_OK) continue;
@@ -382,8 +384,9 @@ int blz_batch_graph_create(blz_ctx* c, const BlzBatchView* views, uint32_t n, bl
     if (!c || !views || n == 0 || !outGraph) return fail(BLZ_ERR_INVALID_ARGUMENT, "bad batch graph arguments");
     *outGraph = nullptr;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    const BlzLaunchShape sh = batch_shape(c, views, n);
-    const uint32_t tile = batch_chunk_for(sh, batch_objects(c, views, n), c->smCount);
+    const uint64_t objectsInAll = batch_objects(c, views, n);
+    const BlzLaunchShape sh = batch_shape(c, objectsInAll, n);
+    const uint32_t tile = batch_chunk_for(sh, objectsInAll, c->smCount);
     std::vector<BatchViewDev> d;
     std::vector<uint32_t> ts;
     int rc = build_views(c, views, n, tile, d, ts);
@@ -413,7 +416,7 @@ int blz_batch_graph_create(blz_ctx* c, const BlzBatchView* views, uint32_t n, bl
             p.scratch = c->scratch;
             if (wants_order(p)) {  // it depends on the lists' sizes alone, which the graph keeps
                 p.order = order;
-                if (launch_batch_order(p, largest_view(ts), order, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
+                if (launch_batch_order(p, order, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
                     rc = fail(BLZ_ERR_CUDA, "batch graph order failed");
             }
         }

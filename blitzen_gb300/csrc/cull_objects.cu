@@ -831,9 +831,9 @@ __global__ void __launch_bounds__(kObjThreads) cull_small_kernel(const PipeParam
     }
 }
 
-// Batched views: two launches. The scan has a block per view: it scans the counts of the view's chunks into
-// {offset in the view's records, view} per chunk and writes the view's draw count (block 0 also rewinds the
-// decide kernel's work counter). The scatter then is one warp per chunk with nothing to wait for. (One launch
+// Batched views: two launches. The scan has a block or a warp per view (batch_scan_by_warps): it scans the counts of
+// the view's chunks into {offset in the view's records, view} per chunk and writes the view's draw count (block 0
+// also rewinds the decide kernel's work counter). The scatter then is one warp per chunk with nothing to wait for. (One launch
 // of 1024-thread blocks, each finding its chunks' views and offsets behind two barriers, took 23 to 30 us for
 // the 33,000 chunks of the 64-view batch, 3.4 waves of them; the two take 3.6 and 14.)
 constexpr uint32_t kBatchScanThreads = 512, kBatchScanEach = 8;
@@ -882,6 +882,48 @@ __global__ void __launch_bounds__(kBatchScanThreads) batch_scan_kernel(const Pip
         const BatchViewDev& bv = p.views[vi];
         *bv.drawCount = carry;
         if (carry > bv.capacity) atomicOr(&p.scratch->status, BLZ_FLAG_COMMAND_OVERFLOW);
+    }
+}
+
+constexpr uint32_t kBatchScanWarpThreads = 256, kBatchScanWarpEach = 8;
+
+// The same with a warp per view, 256 chunks a round, for many views or short ones: a chain of three round trips
+// and no block barrier.
+__global__ void __launch_bounds__(kBatchScanWarpThreads) batch_scan_warp_kernel(const PipeParams p) {
+    constexpr uint32_t EACH = kBatchScanWarpEach;
+    pdl_wait();
+    const uint32_t vi = (blockIdx.x * kBatchScanWarpThreads + threadIdx.x) / 32u, lane = threadIdx.x & 31u;
+    if (blockIdx.x == 0u && threadIdx.x == 0u && p.workCounter != nullptr) *p.workCounter = 0u;
+    if (vi >= p.viewCount) return;
+    const uint32_t first = ldp(p.tileStart + vi), end = ldp(p.tileStart + vi + 1u);
+    const BatchViewDev& bv = p.views[vi];
+    uint32_t* const drawCount = bv.drawCount;
+    const uint32_t capacity = bv.capacity;
+    uint32_t carry = 0;
+    for (uint32_t c0 = first; c0 < end; c0 += 32u * EACH) {
+        uint32_t n[EACH];
+#pragma unroll
+        for (uint32_t k = 0; k < EACH; ++k) {
+            const uint32_t c = c0 + 32u * k + lane;
+            n[k] = c < end ? __ldcg(p.chunkCount + c) : 0u;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < EACH; ++k) {
+            const uint32_t c = c0 + 32u * k + lane;
+            if (c0 + 32u * k >= end) break;  // (the whole warp)
+            uint32_t sum = n[k];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, sum, o);
+                if (lane >= static_cast<uint32_t>(o)) sum += x;
+            }
+            if (c < end) p.chunkBase[c] = make_uint2(carry + sum - n[k], vi);
+            carry += __shfl_sync(0xFFFFFFFFu, sum, 31);
+        }
+    }
+    if (lane == 0u) {
+        *drawCount = carry;
+        if (carry > capacity) atomicOr(&p.scratch->status, BLZ_FLAG_COMMAND_OVERFLOW);
     }
 }
 
@@ -1094,6 +1136,15 @@ static uint32_t scatter_blocks(const PipeParams& p) {
     return n ? n : 1u;
 }
 
+// Whether a batch's chunks are scanned by a warp per view. Views of one round (256 chunks) always are: 2.0 us against
+// 2.9 to 3.9 for up to 256 views, 2.1 against 8.8 for 1,024, 3.3 against 62 for 10,000, since the blocks of the
+// other form take 0.9 us for each view an SM gets. With longer views a round costs 1.2 us: 4,096 views of which one has
+// 16 rounds take 19.8 us against 27.2, 1,024 such 19.7 against 8.9, 2 views of 16 rounds 20.6 against 3.4.
+static bool batch_scan_by_warps(const PipeParams& p, int smCount) {
+    const uint64_t rounds = (p.largest + 32u * kBatchScanWarpEach - 1u) / (32u * kBatchScanWarpEach);
+    return rounds <= 1u || 4u * rounds * static_cast<uint64_t>(smCount > 0 ? smCount : 1) <= 3u * static_cast<uint64_t>(p.viewCount);
+}
+
 template <int MODE, bool SINGLE, int THREADS, int OPT>
 static cudaError_t launch_t(const PipeParams& p, uint32_t blocksPerSm, int smCount, cudaStream_t s) {
     cudaError_t e = launch_decide_t<MODE, SINGLE, THREADS, OPT>(p, blocksPerSm, smCount, s);
@@ -1101,7 +1152,12 @@ static cudaError_t launch_t(const PipeParams& p, uint32_t blocksPerSm, int smCou
     if constexpr (SINGLE) {
         return launch_pdl(cull_scatter_kernel, scatter_blocks(p), kScatterWarps * 32, 0, s, p);
     } else {
-        e = launch_pdl(batch_scan_kernel, p.viewCount, kBatchScanThreads, 0, s, p);
+        if (batch_scan_by_warps(p, smCount)) {
+            constexpr uint32_t views = kBatchScanWarpThreads / 32u;
+            e = launch_pdl(batch_scan_warp_kernel, (p.viewCount + views - 1u) / views, kBatchScanWarpThreads, 0, s, p);
+        } else {
+            e = launch_pdl(batch_scan_kernel, p.viewCount, kBatchScanThreads, 0, s, p);
+        }
         if (e != cudaSuccess) return e;
         constexpr uint32_t per = kBatchScatterThreads / 32u * kBatchScatterChunks;
         return launch_pdl(batch_scatter_kernel, (p.totalTiles + per - 1u) / per, kBatchScatterThreads, 0, s, p);
@@ -1110,9 +1166,9 @@ static cudaError_t launch_t(const PipeParams& p, uint32_t blocksPerSm, int smCou
 
 uint32_t object_tile_size() { return kChunk; }
 
-cudaError_t launch_batch_order(const PipeParams& p, uint32_t largest, uint32_t* order, cudaStream_t s) {
+cudaError_t launch_batch_order(const PipeParams& p, uint32_t* order, cudaStream_t s) {
     return launch_pdl(batch_order_kernel, (p.totalTiles + kBatchOrderThreads - 1u) / kBatchOrderThreads, kBatchOrderThreads, 0, s, p.tileStart, p.viewCount, p.totalTiles,
-                      largest < (1u << 15) ? 1u : 0u, order);
+                      p.largest < (1u << 15) ? 1u : 0u, order);
 }
 
 template <int THREADS, int OPT>

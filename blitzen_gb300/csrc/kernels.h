@@ -119,7 +119,7 @@ struct PipeParams {
     uint32_t* chunkCount2; // fused frame: [totalTiles]
     uint32_t* instHist;    // instanced pass: [groups][lodCount] record counts (zero before the launch)
     uint32_t instLods;     // instanced pass: the histogram's row length (the scene's LOD count)
-    uint32_t pad2;
+    uint32_t largest;      // batches: the most chunks a view has
 };
 
 struct InstancedParams {
@@ -228,7 +228,7 @@ inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, 
 
 uint32_t object_tile_size();
 // The decide order of a batch whose views read a transform table that does not stay in L2 (see
-// batch_order_kernel; p: tileStart, viewCount, totalTiles; largest: the most chunks a view has). Worth its 3 us from tables of kBatchOrderBytes
+// batch_order_kernel; p: tileStart, viewCount, totalTiles, largest). Worth its 3 us from tables of kBatchOrderBytes
 // on; up to kBatchOrderViews views.
 constexpr uint32_t kBatchOrderViews = 256;
 constexpr size_t kBatchOrderBytes = size_t(48) << 20;
@@ -238,7 +238,7 @@ constexpr uint64_t kBatchOrderObjects = uint64_t(1) << 21;
 // 32 23, 18 to 20 and 31, for 64 23, 18 and 31. At 2M objects (32 views) 32 keeps chunks of 512; 64 gained 6% on one
 // pass and lost nothing, but doubles the scratch slots.
 constexpr uint32_t kBatchWarpsPerSm = 32;
-cudaError_t launch_batch_order(const PipeParams& p, uint32_t largest, uint32_t* order, cudaStream_t s);
+cudaError_t launch_batch_order(const PipeParams& p, uint32_t* order, cudaStream_t s);
 // Chunk size of a single-view launch of `count` objects: one chunk per warp the launch holds
 // resident, so every warp streams one contiguous run of objects and none waits for a second round.
 // (Smaller chunks handed out by a counter measured slower: each chunk drains its survivor ring in
