@@ -13,7 +13,7 @@
 //            documented form (VendorCode/Meshoptimizer/meshoptimizer.h:561-569). A visible cluster
 //            sets its bit in the tile's slot-ordered visibility words and counts towards its tile
 //            and the frame;
-//   emit     one warp per tile with records: the records of the tiles before it (from the counts
+//   emit     1, 4 or 8 warps per tile with records (emit_warps): the records of the tiles before it (from the counts
 //            per group of 64 tiles, which the test launch also keeps), then a record for every set
 //            bit at its final position, without repeating a test.
 // Nothing is materialised per candidate cluster but its bit.
@@ -33,7 +33,6 @@ constexpr int kClWarps = kClThreads / 32;
 constexpr uint32_t kClObjects = 32;  // objects per tile
 constexpr uint32_t kClItem = 64;     // clusters per work item of the test launch (two per lane)
 constexpr uint32_t kClSuper = 64;     // tiles per group whose counts the test launch also sums
-constexpr uint32_t kClEmitWarps = 8;     // emit launch: warps per tile (2: 8.4 us, 4: 6.2, 8: 5.2 for 12,345 objects in task form)
 constexpr uint32_t kClPrefixLoads = 4;   // emit launch: group and tile counts each lane loads at once
 
 // Sphere, Hi-Z and cone tests of one cluster of an object. The int8 cone axis and cutoff are divided
@@ -238,19 +237,18 @@ __global__ void __launch_bounds__(kClThreads) cluster_test_kernel(const ClusterP
     }
 }
 
-// Emit launch, kClEmitWarps warps per tile (lane = object): no test is repeated. The last tile's first warp
+// Emit launch, EW warps per tile (lane = object; emit_warps): no test is repeated. The last tile's first warp
 // writes the frame's counts; a tile without records returns. The tile's warps take its set bits 32 at a
-// time in turn: a view of few objects has few tiles (12,345 objects: 386 on 152 SMs, some 360 records
-// each), and one warp per tile took 11 to 13 us there against 5.2. The tile's cluster ranges, visibility bits
+// time in turn. The tile's cluster ranges, visibility bits
 // and counts come from the earlier launches, the records (task form: tasks and payloads) before it
 // from the counts of the groups of tiles before its group and of the tiles of its group before it;
 // every set bit is written at its final position in slot order, the tile's set bits spread over
 // the lanes 32 at a time.
-template <bool TASKS>
+template <bool TASKS, uint32_t EW>
 __global__ void __launch_bounds__(kClThreads) cluster_emit_kernel(const ClusterParams p) {
     pdl_wait();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t tile = (blockIdx.x * kClWarps + warp) / kClEmitWarps, part = warp % kClEmitWarps;
+    const uint32_t tile = (blockIdx.x * kClWarps + warp) / EW, part = warp % EW;
     if (tile >= p.tiles) return;
     const uint32_t lt = lanemask_lt();
     const uint32_t* bits = p.bits + static_cast<size_t>(tile) * p.bitWords;
@@ -337,8 +335,14 @@ __global__ void __launch_bounds__(kClThreads) cluster_emit_kernel(const ClusterP
                 tw[3] = 1u;
             }
         }
-        // the last payload's unused slots, an object at a time, a slot per lane
-        for (uint32_t o = part; o < kClObjects; o += kClEmitWarps) {
+        // the last payload's unused slots: by the object's lane, or an object at a time, a slot per lane
+        if constexpr (EW == 1u) {
+            const uint32_t last = first + k - 1u;
+            if ((sv & 31u) != 0u && last < p.payloadCapacity) {
+                uint32_t* pw = p.payloads + static_cast<size_t>(last) * 33u + 1u;
+                for (uint32_t e = sv & 31u; e < 32u; ++e) pw[e] = BLZ_NO_MESHLET;
+            }
+        } else for (uint32_t o = part; o < kClObjects; o += EW) {
             const uint32_t so = __shfl_sync(0xFFFFFFFFu, sv, static_cast<int>(o));
             const uint32_t last = __shfl_sync(0xFFFFFFFFu, first + k - 1u, static_cast<int>(o));
             if ((so & 31u) != 0u && lane >= (so & 31u) && last < p.payloadCapacity)
@@ -361,7 +365,7 @@ __global__ void __launch_bounds__(kClThreads) cluster_emit_kernel(const ClusterP
         }
         const uint32_t wexcl = wincl - c;
         const uint32_t roundTotal = __shfl_sync(0xFFFFFFFFu, wincl, 31);
-        for (uint32_t k0 = part * 32u; k0 < roundTotal; k0 += 32u * kClEmitWarps) {
+        for (uint32_t k0 = part * 32u; k0 < roundTotal; k0 += 32u * EW) {
             const uint32_t k = k0 + lane;  // the round's set bit taken by this lane
             uint32_t j = 0;                // its word: the number of words with wincl <= k
 #pragma unroll
@@ -405,6 +409,28 @@ uint32_t cluster_tile_objects() { return kClObjects; }
 
 uint32_t cluster_tile_groups(uint32_t tiles) { return (tiles + kClSuper - 1) / kClSuper; }
 
+// Warps per tile of the emit launch. Each of them sums the counts before the tile and scans its words for itself, so
+// more than one pays only where the tiles alone leave the chip idle (12,345 objects are 386 tiles, on 152 SMs) and
+// have records for all of them; a tile's words of visibility bits, one per cluster of the longest LOD, bound its
+// records by 32 each. us a launch with 1, 4 and 8 warps, every object's clusters in view:
+//   objects x clusters      1      4      8
+//     2,000 x 100        13.3    6.4    5.3
+//    12,345 x 4           3.0    3.3    3.6
+//    12,345 x 20          4.9    3.5    3.8
+//    12,345 x 120        14.8    7.7    6.1
+//    25,000 x 40          6.9    4.9    5.0
+//    50,000 x 8           4.0    5.3    6.9
+//    50,000 x 200        27.0   16.7   14.9
+//   100,000 x 100        18.0   15.2   16.4
+//   200,000 x 60         15.1   19.8   27.8
+// 1,000,000 x 4          47.8    170    327
+// (as many objects, none in view: 3.5, 10.2 and 19.4 us). The lines below are where these cross.
+static uint32_t emit_warps(const ClusterParams& p) {
+    for (uint32_t w : {8u, 4u})
+        if (p.bitWords >= 5u * w && static_cast<uint64_t>(p.tiles) * w <= 160ull * p.bitWords) return w;
+    return 1u;
+}
+
 template <bool TASKS>
 static cudaError_t launch_cluster(const ClusterParams& p, const BlzCameraViewData& view, cudaStream_t s) {
     const uint32_t tileBlocks = (p.tiles + kClWarps - 1) / kClWarps;
@@ -416,7 +442,11 @@ static cudaError_t launch_cluster(const ClusterParams& p, const BlzCameraViewDat
     blocks = std::min<uint64_t>(blocks, (maxItems + kClWarps - 1) / kClWarps);
     e = launch_pdl(cluster_test_kernel<TASKS>, static_cast<uint32_t>(blocks ? blocks : 1), kClThreads, 0, s, p, view);
     if (e != cudaSuccess) return e;
-    return launch_pdl(cluster_emit_kernel<TASKS>, (p.tiles * kClEmitWarps + kClWarps - 1) / kClWarps, kClThreads, 0, s, p);
+    const uint32_t ew = emit_warps(p);
+    const uint32_t emitBlocks = (p.tiles * ew + kClWarps - 1) / kClWarps;
+    if (ew == 8u) return launch_pdl(cluster_emit_kernel<TASKS, 8>, emitBlocks, kClThreads, 0, s, p);
+    if (ew == 4u) return launch_pdl(cluster_emit_kernel<TASKS, 4>, emitBlocks, kClThreads, 0, s, p);
+    return launch_pdl(cluster_emit_kernel<TASKS, 1>, emitBlocks, kClThreads, 0, s, p);
 }
 
 cudaError_t cluster_test_blocks_per_sm(bool tasks, int* out) {
