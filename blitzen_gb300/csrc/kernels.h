@@ -290,10 +290,11 @@ cudaError_t launch_transforms_rotate(const BlzMeshTransform* table, uint32_t tab
 cudaError_t launch_add_word(unsigned int* word, unsigned int n, cudaStream_t s);
 // *out = atomicExch(status, 0) on the stream (one thread).
 cudaError_t launch_take_status(unsigned int* status, unsigned int* out, cudaStream_t s);
-// Up to this many boxes are rasterised by screen tiles (each tile reads every box's rectangle, from
+// Up to this many boxes are rasterised by screen tiles (a tile reads the rectangles of every box, or of its bin, from
 // rectScratch, kRasterScratchBytes of the context's memory), more by a block per box and atomic maxima.
 constexpr uint32_t kRasterTileBoxes = 8192;
-constexpr size_t kRasterScratchBytes = size_t(kRasterTileBoxes) * 20;
+constexpr uint32_t kRasterBinSide = 16;  // bins across and down the screen at most, a bit per box each
+constexpr size_t kRasterScratchBytes = size_t(kRasterTileBoxes) * 20 + size_t(kRasterBinSide) * kRasterBinSide * (kRasterTileBoxes / 8);
 cudaError_t launch_depth_raster(const BlzCameraViewData& view, const float* boxes, uint32_t boxCount, float* depth,
                                 uint32_t width, uint32_t height, void* rectScratch, cudaStream_t s, uint32_t* launches);
 

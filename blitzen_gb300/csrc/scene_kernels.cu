@@ -150,8 +150,8 @@ __global__ void depth_raster_kernel(const BlzCameraViewData view, const float* b
 // writes the pixel once, the cleared ones included: the image is written once and never read, where the
 // block per box clears it and then sends one atomic a covered pixel.
 // 2000 boxes of the stress scene's sizes at 3840x2160: 13 us a raster (2.8 rectangles, 12.0 tiles, in a
-// stream) against 32; 8192 boxes of 1 to 4 units there, the tile form's worst: 25 against 28, and
-// since a tile tests every box, that is where the dispatch's line lies.
+// stream) against 32; 8192 boxes of 1 to 4 units, the tile form's worst: 15 against 37, and 177 against 195 at
+// 16384x16384, where most of either is the writing of the image.
 constexpr uint32_t kTileW = 64, kTileH = 64;  // (128 x 64: 16.1 us a tile launch against 12.0: a warp meets more boxes it has no pixel of)
 constexpr uint32_t kTileThreads = kTileW / 4u * kTileH / 4u;
 constexpr uint32_t kTileHits = 1024;
@@ -198,8 +198,30 @@ __global__ void __launch_bounds__(128) box_rects_kernel(const BlzCameraViewData 
     depths[b] = __float_as_int(r.depth);
 }
 
+// Bins of the screen, kRasterBinSide by kRasterBinSide at most, whole tiles each: a block per bin marks the boxes
+// that meet it, a bit each, so that a tile tests the boxes of its bin and not all of them.
+constexpr uint32_t kBinThreads = 1024;
+constexpr uint32_t kBinWords = kRasterTileBoxes / 32u;
+static_assert(kBinWords <= kTileThreads, "a word of the bin's boxes per thread of a tile");
+
+__global__ void __launch_bounds__(kBinThreads) box_bins_kernel(const int4* rects, uint32_t boxCount, uint32_t binW, uint32_t binH,
+                                                               uint32_t* masks) {
+    pdl_wait();
+    const int X0 = static_cast<int>(blockIdx.x * binW), Y0 = static_cast<int>(blockIdx.y * binH);
+    const int X1 = X0 + static_cast<int>(binW), Y1 = Y0 + static_cast<int>(binH);
+    uint32_t* const mask = masks + static_cast<size_t>(blockIdx.y * gridDim.x + blockIdx.x) * kBinWords;
+    for (uint32_t first = 0; first < boxCount; first += kBinThreads) {
+        const uint32_t b = first + threadIdx.x;
+        const int4 r = b < boxCount ? rects[b] : make_int4(0, 0, 0, 0);  // (empty, as those of boxes not drawn)
+        const uint32_t word = __ballot_sync(0xFFFFFFFFu, r.z > r.x && r.x < X1 && r.z > X0 && r.y < Y1 && r.w > Y0);
+        if (threadIdx.x % 32u == 0u && b < boxCount) mask[b / 32u] = word;
+    }
+}
+
+template <bool BINS>
 __global__ void __launch_bounds__(kTileThreads) depth_tiles_kernel(const int4* rects, const int* depths, uint32_t boxCount,
-                                                                   float* depth, uint32_t width, uint32_t height, uint32_t vec4) {
+                                                                   float* depth, uint32_t width, uint32_t height, uint32_t vec4,
+                                                                   const uint32_t* masks, uint32_t binW, uint32_t binH, uint32_t binsX) {
     __shared__ int4 s_rect[kTileHits];
     __shared__ int s_depth[kTileHits];
     __shared__ uint32_t s_hits;
@@ -213,7 +235,61 @@ __global__ void __launch_bounds__(kTileThreads) depth_tiles_kernel(const int4* r
     for (int j = 0; j < 4; ++j)
 #pragma unroll
         for (int i = 0; i < 4; ++i) v[j][i] = 0;
-    for (uint32_t first = 0; first < boxCount; first += kTileThreads * kTileScan) {
+    auto meets = [&](const int4& q) {
+        return q.x < X0 + static_cast<int>(kTileW) && q.z > X0 && q.y < Y0 + static_cast<int>(kTileH) && q.w > Y0;
+    };
+    auto keep = [&](const int4& q, uint32_t b) {
+        const uint32_t at = atomicAdd(&s_hits, 1u);
+        s_rect[at] = q;
+        s_depth[at] = depths[b];
+    };
+    auto draw_list = [&] {
+        const uint32_t n = s_hits;
+        for (uint32_t h = 0; h < n; ++h) {
+            const int4 q = s_rect[h];
+            if (q.x >= wx + 32 || q.z <= wx || q.y >= wy + 16 || q.w <= wy) continue;  // (the whole warp)
+            const int d = s_depth[h];
+            int c[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) c[i] = x + i >= q.x && x + i < q.z ? d : 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int row = y + 4 * j;
+                if (row >= q.y && row < q.w) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) v[j][i] = max(v[j][i], c[i]);
+                }
+            }
+        }
+    };
+    bool all = true;  // whether every box is tested
+    if constexpr (BINS) {
+        // the boxes of the tile's bin, when the list holds them: at most kTileHits, tested in one go
+        __shared__ uint16_t s_bin[kTileHits];
+        __shared__ uint32_t s_marked;
+        const uint32_t bin = static_cast<uint32_t>(Y0) / binH * binsX + static_cast<uint32_t>(X0) / binW;
+        uint32_t word = threadIdx.x * 32u < boxCount ? masks[static_cast<size_t>(bin) * kBinWords + threadIdx.x] : 0u;
+        if (threadIdx.x == 0) s_hits = s_marked = 0u;
+        __syncthreads();
+        if (word != 0u) {
+            uint32_t at = atomicAdd(&s_marked, static_cast<uint32_t>(__popc(word)));
+            for (; word != 0u && at < kTileHits; word &= word - 1u)
+                s_bin[at++] = static_cast<uint16_t>(threadIdx.x * 32u + static_cast<uint32_t>(__ffs(static_cast<int>(word)) - 1));
+        }
+        __syncthreads();
+        const uint32_t marked = s_marked;
+        all = marked > kTileHits;
+        if (!all) {
+            for (uint32_t i = threadIdx.x; i < marked; i += kTileThreads) {
+                const uint32_t b = s_bin[i];
+                const int4 q = rects[b];
+                if (meets(q)) keep(q, b);
+            }
+            __syncthreads();
+            draw_list();
+        }
+    }
+    for (uint32_t first = 0; all && first < boxCount; first += kTileThreads * kTileScan) {
         int4 r[kTileScan];
 #pragma unroll
         for (uint32_t k = 0; k < kTileScan; ++k) {
@@ -228,30 +304,10 @@ __global__ void __launch_bounds__(kTileThreads) depth_tiles_kernel(const int4* r
             __syncthreads();
 #pragma unroll
             for (uint32_t k = part; k < part + kTilePart; ++k) {
-                if (r[k].x < X0 + static_cast<int>(kTileW) && r[k].z > X0 && r[k].y < Y0 + static_cast<int>(kTileH) && r[k].w > Y0) {
-                    const uint32_t at = atomicAdd(&s_hits, 1u);
-                    s_rect[at] = r[k];
-                    s_depth[at] = depths[first + k * kTileThreads + threadIdx.x];
-                }
+                if (meets(r[k])) keep(r[k], first + k * kTileThreads + threadIdx.x);
             }
             __syncthreads();
-            const uint32_t n = s_hits;
-            for (uint32_t h = 0; h < n; ++h) {
-                const int4 q = s_rect[h];
-                if (q.x >= wx + 32 || q.z <= wx || q.y >= wy + 16 || q.w <= wy) continue;  // (the whole warp)
-                const int d = s_depth[h];
-                int c[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) c[i] = x + i >= q.x && x + i < q.z ? d : 0;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int row = y + 4 * j;
-                    if (row >= q.y && row < q.w) {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) v[j][i] = max(v[j][i], c[i]);
-                    }
-                }
-            }
+            draw_list();
         }
     }
 #pragma unroll
@@ -269,6 +325,16 @@ __global__ void __launch_bounds__(kTileThreads) depth_tiles_kernel(const int4* r
     }
 }
 
+// Whether the boxes are sorted into bins first. A tile without bins loads 1,024 rectangles a round, so up to there is
+// nothing to save (1,000 tiny boxes at 16384x16384: 144 us, 155 with bins; 2,000: 184 and 164), and the bins' launch
+// costs 2 to 3 us. us a raster without and with them, boxes of 1 to 4 units and of 10 to 200:
+//   2,000 boxes, 3840x2160    11.0  11.5   |  13.5  13.5
+//   3,000 boxes, 3840x2160    13.2  12.4   |  17.4  15.7
+//   8,192 boxes, 3840x2160    25.4  14.9   |  36.0  24.8
+//   8,192 boxes, 8192x8192     140    56   |   185    88
+//   8,192 boxes, 16384x16384   546   177   |   691   305
+static bool raster_bins(uint32_t boxCount, uint64_t tiles) { return boxCount > 1536u && boxCount * tiles >= 5'000'000u; }
+
 cudaError_t launch_depth_raster(const BlzCameraViewData& view, const float* boxes, uint32_t boxCount, float* depth,
                                 uint32_t width, uint32_t height, void* rectScratch, cudaStream_t s, uint32_t* launches) {
     if (boxCount > 0 && boxCount <= kRasterTileBoxes && width <= kRasterTileExtent && height <= kRasterTileExtent) {
@@ -278,11 +344,18 @@ cudaError_t launch_depth_raster(const BlzCameraViewData& view, const float* boxe
         if (e != cudaSuccess) return e;
         const dim3 grid((width + kTileW - 1) / kTileW, (height + kTileH - 1) / kTileH);
         const uint32_t vec4 = width % 4u == 0u && reinterpret_cast<uintptr_t>(depth) % 16 == 0 ? 1u : 0u;
-        e = launch_pdl(depth_tiles_kernel, grid, kTileThreads, 0, s, static_cast<const int4*>(rects), static_cast<const int*>(depths),
-                       boxCount, depth, width, height, vec4);
-        if (e != cudaSuccess) return e;
         if (launches) *launches += 2;
-        return cudaSuccess;
+        if (!raster_bins(boxCount, static_cast<uint64_t>(grid.x) * grid.y))
+            return launch_pdl(depth_tiles_kernel<false>, grid, kTileThreads, 0, s, static_cast<const int4*>(rects), static_cast<const int*>(depths),
+                              boxCount, depth, width, height, vec4, static_cast<const uint32_t*>(nullptr), 0u, 0u, 0u);
+        if (launches) *launches += 1;
+        uint32_t* masks = reinterpret_cast<uint32_t*>(depths + kRasterTileBoxes);
+        const uint32_t binW = (grid.x + kRasterBinSide - 1) / kRasterBinSide * kTileW, binH = (grid.y + kRasterBinSide - 1) / kRasterBinSide * kTileH;
+        const dim3 bins((width + binW - 1) / binW, (height + binH - 1) / binH);
+        e = launch_pdl(box_bins_kernel, bins, kBinThreads, 0, s, static_cast<const int4*>(rects), boxCount, binW, binH, masks);
+        if (e != cudaSuccess) return e;
+        return launch_pdl(depth_tiles_kernel<true>, grid, kTileThreads, 0, s, static_cast<const int4*>(rects), static_cast<const int*>(depths),
+                          boxCount, depth, width, height, vec4, static_cast<const uint32_t*>(masks), binW, binH, bins.x);
     }
     const size_t n = static_cast<size_t>(width) * height;
     const size_t n4 = (reinterpret_cast<uintptr_t>(depth) % 16 == 0) ? n / 4 : 0;
