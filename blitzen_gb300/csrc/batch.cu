@@ -59,11 +59,30 @@ static BlzLaunchShape batch_shape(const blz_ctx* c, uint64_t objects, uint32_t n
     return t ? t->shape : c->shape;
 }
 
-static int build_views(blz_ctx* c, const BlzBatchView* views, uint32_t n, uint32_t tile, std::vector<BatchViewDev>& out,
-                       std::vector<uint32_t>& tileStart) {
+// The pass all views run, or -1 when they differ.
+static int uniform_mode(const BlzBatchView* views, uint32_t n) {
+    for (uint32_t i = 1; i < n; ++i)
+        if (views[i].mode != views[0].mode) return -1;
+    return n ? static_cast<int>(views[0].mode) : -1;
+}
+
+// Place of each view among the device's: those of one pass together, in the caller's order, since the warps of an SM
+// that run different passes at a time thrash its instruction cache.
+static std::vector<uint32_t> pass_places(const BlzBatchView* views, uint32_t n) {
+    uint32_t next[BLZ_MODE_TEMPORAL + 2] = {};  // (any mode past the last is refused where the view is built)
+    auto pass = [&](uint32_t i) { return std::min<uint32_t>(views[i].mode, BLZ_MODE_TEMPORAL + 1); };
+    for (uint32_t i = 0; i < n; ++i)
+        for (uint32_t m = pass(i) + 1; m < BLZ_MODE_TEMPORAL + 2; ++m) ++next[m];
+    std::vector<uint32_t> place(n);
+    for (uint32_t i = 0; i < n; ++i) place[i] = next[pass(i)]++;
+    return place;
+}
+
+// The device's views and the first chunk of each. place: where each view goes, or empty: in the caller's order.
+static int build_views(blz_ctx* c, const BlzBatchView* views, uint32_t n, uint32_t tile, const std::vector<uint32_t>& place,
+                       std::vector<BatchViewDev>& out, std::vector<uint32_t>& tileStart) {
     out.resize(n);
     tileStart.resize(n + 1);
-    uint64_t at = 0;
     for (uint32_t i = 0; i < n; ++i) {
         const BlzBatchView& v = views[i];
         if (v.mode > BLZ_MODE_TEMPORAL) return fail(BLZ_ERR_INVALID_ARGUMENT, "view %u: unknown mode %u", i, v.mode);
@@ -95,9 +114,12 @@ static int build_views(blz_ctx* c, const BlzBatchView* views, uint32_t n, uint32
         d.drawCount = v.target.drawCount;
         d.dynT = v.dynamicTransforms;
         d.dynCount = v.dynamicCount;
-        out[i] = d;
+        out[place.empty() ? i : place[i]] = d;
+    }
+    uint64_t at = 0;
+    for (uint32_t i = 0; i < n; ++i) {
         tileStart[i] = static_cast<uint32_t>(at);
-        uint64_t tiles = (count + tile - 1) / tile;
+        uint64_t tiles = (out[i].count + tile - 1) / tile;
         if (tiles == 0) tiles = 1;  // an empty view still gets one item that writes drawCount = 0
         at += tiles;
     }
@@ -154,25 +176,20 @@ static int ensure_batch_dev(blz_ctx* c, size_t bytes) {
     return BLZ_OK;
 }
 
-// The pass all views run, or -1 when they differ.
-static int uniform_mode(const BlzBatchView* views, uint32_t n) {
-    for (uint32_t i = 1; i < n; ++i)
-        if (views[i].mode != views[0].mode) return -1;
-    return n ? static_cast<int>(views[0].mode) : -1;
-}
-
-// Whether the chunks are decided in the order of batch_order_kernel: several views, enough chunks for it to
-// matter, and a transform table that would be read from memory again for each view.
-static bool wants_order(const PipeParams& p) {
-    return p.viewCount > 1 && p.viewCount <= kBatchOrderViews && static_cast<uint64_t>(p.totalTiles) * p.chunkSize >= kBatchOrderObjects &&
+// Whether the chunks are decided in the order of batch_order_kernel: several views, all of one pass (the order would
+// mix the passes, see pass_places), enough chunks for it to matter, and a transform table that would be read from
+// memory again for each view.
+static bool wants_order(const PipeParams& p, int mode) {
+    return mode >= 0 && p.viewCount > 1 && p.viewCount <= kBatchOrderViews && static_cast<uint64_t>(p.totalTiles) * p.chunkSize >= kBatchOrderObjects &&
            p.sc.transformCount * sizeof(BlzMeshTransform) >= kBatchOrderBytes;
 }
 
 static int run_batch_shape(blz_ctx* c, const BlzBatchView* views, uint32_t n, uint64_t objects, cudaStream_t st, const BlzLaunchShape& sh) {
     const uint32_t tile = batch_chunk_for(sh, objects, c->smCount);
+    const int mode = uniform_mode(views, n);
     std::vector<BatchViewDev> d;
     std::vector<uint32_t> ts;
-    int rc = build_views(c, views, n, tile, d, ts);
+    int rc = build_views(c, views, n, tile, mode < 0 ? pass_places(views, n) : std::vector<uint32_t>(), d, ts);
     if (rc != BLZ_OK) return rc;
     rc = ensure_batch_dev(c, batch_bytes(n));
     if (rc != BLZ_OK) return rc;
@@ -183,14 +200,14 @@ static int run_batch_shape(blz_ctx* c, const BlzBatchView* views, uint32_t n, ui
     if (rc != BLZ_OK) return rc;
     bind_chunk_scratch(c, p);
     cudaError_t e = cudaSuccess;
-    if (wants_order(p)) {
+    if (wants_order(p, mode)) {
         uint32_t* order = p.chunkCount + c->chunkSlots;
         e = launch_batch_order(p, order, st);
         p.order = order;
         c->launches++;
     }
     if (e == cudaSuccess)
-        e = launch_batch_cull(p, sh.threadsPerBlock, sh.objectsPerThread, sh.blocksPerSm, c->smCount, st, uniform_mode(views, n));
+        e = launch_batch_cull(p, sh.threadsPerBlock, sh.objectsPerThread, sh.blocksPerSm, c->smCount, st, mode);
     if (e != cudaSuccess) return cuda_fail(e, "batch launch");
     c->launches += 3;  // decide, scan, scatter
     return BLZ_OK;
@@ -212,6 +229,7 @@ struct blz_batch_graph {
     void* viewsDev = nullptr;
     void* chunkMem = nullptr;  // the graph's own staging scratch (a context's may be reallocated)
     uint32_t viewCount = 0;
+    std::vector<uint32_t> place;  // where each view lies among the device's, or empty: in order
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
 };
@@ -280,7 +298,7 @@ int blz_cull_batch_per_view(blz_ctx* c, const BlzBatchView* views, uint32_t n, b
     std::vector<BatchViewDev> d;
     std::vector<uint32_t> ts;
     const uint32_t tile = batch_chunk(batch_shape(c, batch_objects(c, views, n), n));
-    int rc = build_views(c, views, n, tile, d, ts);
+    int rc = build_views(c, views, n, tile, {}, d, ts);  // launched one by one, in the caller's order
     if (rc != BLZ_OK) return rc;
     uint32_t maxTiles = 1;
     for (uint32_t i = 0; i < n; ++i) maxTiles = std::max(maxTiles, ts[i + 1] - ts[i]);
@@ -387,11 +405,15 @@ int blz_batch_graph_create(blz_ctx* c, const BlzBatchView* views, uint32_t n, bl
     const uint64_t objectsInAll = batch_objects(c, views, n);
     const BlzLaunchShape sh = batch_shape(c, objectsInAll, n);
     const uint32_t tile = batch_chunk_for(sh, objectsInAll, c->smCount);
+    const int mode = uniform_mode(views, n);
+    std::vector<uint32_t> place;
+    if (mode < 0) place = pass_places(views, n);
     std::vector<BatchViewDev> d;
     std::vector<uint32_t> ts;
-    int rc = build_views(c, views, n, tile, d, ts);
+    int rc = build_views(c, views, n, tile, place, d, ts);
     if (rc != BLZ_OK) return rc;
     blz_batch_graph* g = new blz_batch_graph();
+    g->place = place;
     g->ctx = c;
     g->viewCount = n;
     if (cudaMalloc(&g->viewsDev, batch_bytes(n)) != cudaSuccess) {
@@ -414,7 +436,7 @@ int blz_batch_graph_create(blz_ctx* c, const BlzBatchView* views, uint32_t n, bl
             uint32_t* order = p.chunkCount + chunks;
             p.workCounter = reinterpret_cast<unsigned int*>(order + chunks);  // zeroed above
             p.scratch = c->scratch;
-            if (wants_order(p)) {  // it depends on the lists' sizes alone, which the graph keeps
+            if (wants_order(p, mode)) {  // it depends on the lists' sizes alone, which the graph keeps
                 p.order = order;
                 if (launch_batch_order(p, order, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
                     rc = fail(BLZ_ERR_CUDA, "batch graph order failed");
@@ -426,8 +448,7 @@ int blz_batch_graph_create(blz_ctx* c, const BlzBatchView* views, uint32_t n, bl
         cudaError_t e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            cudaError_t le = launch_batch_cull(p, sh.threadsPerBlock, sh.objectsPerThread, sh.blocksPerSm, c->smCount, cap,
-                                               uniform_mode(views, n));
+            cudaError_t le = launch_batch_cull(p, sh.threadsPerBlock, sh.objectsPerThread, sh.blocksPerSm, c->smCount, cap, mode);
             e = cudaStreamEndCapture(cap, &g->graph);
             if (le != cudaSuccess) e = le;
         }
@@ -445,7 +466,8 @@ int blz_batch_graph_create(blz_ctx* c, const BlzBatchView* views, uint32_t n, bl
 
 int blz_batch_graph_set_view(blz_batch_graph* g, uint32_t i, const BlzCameraViewData* view) {
     if (!g || !view || i >= g->viewCount) return fail(BLZ_ERR_INVALID_ARGUMENT, "bad batch graph view update");
-    char* dst = static_cast<char*>(g->viewsDev) + sizeof(BatchViewDev) * i + offsetof(BatchViewDev, view);
+    const uint32_t at = g->place.empty() ? i : g->place[i];
+    char* dst = static_cast<char*>(g->viewsDev) + sizeof(BatchViewDev) * at + offsetof(BatchViewDev, view);
     cudaError_t e = cudaMemcpy(dst, view, sizeof(BlzCameraViewData), cudaMemcpyHostToDevice);
     return e == cudaSuccess ? BLZ_OK : cuda_fail(e, "batch graph view update");
 }

@@ -66,12 +66,15 @@ constexpr uint32_t kChunk = 512;  // objects per chunk of batched views, unless 
 constexpr uint32_t kInstGroup = 32;
 
 // Where the reject test (surely_outside) comes before the exact frustum test, and the exact test runs in the
-// dense stage, on the objects the bound cannot drop: the one-call frame and batched views. The frame of 4M
-// objects took 52.3 us without and 48.8 with it, a batch of 64 views 300 and 287. The other
+// dense stage, on the objects the bound cannot drop: the one-call frame and batches whose views all run one pass. The
+// frame of 4M objects took 52.3 us without and 48.8 with it, a batch of 64 views 300 and 287. The other
 // single-view passes test every object exactly where it is loaded: most of their lists are short or, in
 // pass 1, mostly inside the frustum, and the second stage's latency cost 0.2 to 0.9 us of passes of 100k to
-// 1M objects (at 4M the instanced pass gained 0.2 us).
-__host__ __device__ constexpr bool reject_mode(int mode, bool single) { return !single || mode == 5 || mode == 6; }
+// 1M objects (at 4M the instanced pass gained 0.2 us). The kernel that reads each view's pass holds the code of all four, which the bound makes longer: with it 32 views of 500,000 objects, 8 of each pass, took 185 us at
+// two objects a thread and 307 at four against 169 and 256 without; with one object a thread it is 160 against 221.
+__host__ __device__ constexpr bool reject_mode(int mode, bool single, int opt) {
+    return single ? mode == 5 || mode == 6 : mode != kModeRuntime || opt == 1;
+}
 static_assert(kModeFrameFused == 5 && kModeFramePyr == 6, "reject_mode names the fused modes");
 
 // A warp's queue of objects waiting for the dense stage, in shared memory.
@@ -273,15 +276,15 @@ __host__ __device__ constexpr uint32_t candidate_slots(int mode, bool single, in
 //      (REJECT: the exact frustum test; projection, Hi-Z, LOD) never runs on a lane without an object;
 //   3  the dense stage stages the emitted ones in order; the rest drains at the end.
 // Returns the number of records staged. No block barrier: warps never wait for one another.
-template <int MODE, bool SINGLE, int OPT>
+template <int MODE, bool SINGLE, int OPT, bool REJECT>
 __device__ __forceinline__ uint32_t decide_run_warp(const SceneTables& sc, const BatchViewDev& bv, uint32_t base,
-                                                    uint32_t limit, uint2* stage, Ring<reject_mode(MODE, SINGLE)>& ring, Candidates<candidate_slots(MODE, SINGLE, OPT)>& cand,
+                                                    uint32_t limit, uint2* stage, Ring<REJECT>& ring, Candidates<candidate_slots(MODE, SINGLE, OPT)>& cand,
                                                     const SurfaceCache& surf, SharedView* shared, unsigned int& flags, uint4* keep,
                                                     uint32_t& kept, uint2* stage1 = nullptr, uint32_t* run1 = nullptr,
                                                     const unsigned int* ready = nullptr, uint32_t spinLimit = 0u,
                                                     uint32_t* hist = nullptr) {
     constexpr uint32_t STEP = 32u * OPT;
-    constexpr bool REJECT = reject_mode(MODE, SINGLE);
+    constexpr bool OWN = SINGLE || !REJECT;  // the view's constants in registers
     constexpr bool PACK = (MODE == BLZ_MODE_FIRST) && SINGLE;  // candidate ring of 2 * STEP entries
     // Single-view pass 2 walks its chunk from the last object down: pass 1 walked the same chunk
     // upwards just before (with only the pyramid build between), so the lines it touched last are
@@ -304,7 +307,7 @@ __device__ __forceinline__ uint32_t decide_run_warp(const SceneTables& sc, const
     // The view's constants: a single view's come from the launch parameters, whose reads are operands of the
     // arithmetic; a batch's are kept in shared memory by the warp and read again by each step and each
     // dense round, since together with the loop's state they do not fit the registers.
-    if constexpr (!SINGLE) {
+    if constexpr (!OWN) {
         __syncwarp();  // the chunk before this one is done with them
         if (threadIdx.x % 32u == 0u) {
             shared->v = load_view(bv.view);
@@ -314,12 +317,12 @@ __device__ __forceinline__ uint32_t decide_run_warp(const SceneTables& sc, const
     }
     ViewConsts own;
     RejectBounds ownRj;
-    if constexpr (SINGLE) {
+    if constexpr (OWN) {
         own = load_view(bv.view);
         ownRj = reject_bounds(own);
     }
-    const ViewConsts& v = SINGLE ? own : shared->v;
-    [[maybe_unused]] const RejectBounds& rj = SINGLE ? ownRj : shared->rj;
+    const ViewConsts& v = OWN ? own : shared->v;
+    [[maybe_unused]] const RejectBounds& rj = OWN ? ownRj : shared->rj;
     // what the loop reads of the view, kept in registers (a batch's views lie in global memory, from where
     // every field would be read again after each store)
     const uint2* const objects = reinterpret_cast<const uint2*>(bv.objects);
@@ -516,15 +519,16 @@ template <int MODE, bool SINGLE, int THREADS, int OPT>
 struct DecideSmem {
     static constexpr int NW = THREADS / 32;
     using Cand = Candidates<candidate_slots(MODE, SINGLE, OPT)>;
-    using Queue = Ring<reject_mode(MODE, SINGLE)>;
-    static constexpr size_t kUsed = (sizeof(Queue) + sizeof(Cand) + (SINGLE ? 0 : sizeof(SharedView))) * NW + sizeof(SharedView);
-    static constexpr bool REJECT = reject_mode(MODE, SINGLE);
+    using Queue = Ring<reject_mode(MODE, SINGLE, OPT)>;
+    static constexpr bool REJECT = reject_mode(MODE, SINGLE, OPT);
+    static constexpr uint32_t kViews = SINGLE || !REJECT ? 1u : NW;
+    static constexpr size_t kUsed = (sizeof(Queue) + sizeof(Cand)) * NW + kViews * sizeof(SharedView);
     static constexpr uint32_t kLods = REJECT && kUsed + 2048 + 1024 <= 48 * 1024 ? 512u : 1u;  // LOD errors
     static constexpr size_t kLeft = kUsed + kLods * 4 + 1024 < 48 * 1024 ? 48 * 1024 - 1024 - kLods * 4 - kUsed : 0;
     static constexpr size_t kSurfBytes = (REJECT ? sizeof(float2) : 0) + sizeof(float4) + sizeof(uint2);
     static constexpr uint32_t kSurf = kLeft >= 512 * kSurfBytes ? 512u : (kLeft >= 256 * kSurfBytes ? 256u : (kLeft >= 64 * kSurfBytes ? 64u : 1u));
     Queue ring[NW];
-    SharedView view[SINGLE ? 1 : NW];
+    SharedView view[kViews];
     Cand cand[NW];
     float4 sphere[kSurf];
     float2 bound[REJECT ? kSurf : 1u];
@@ -590,7 +594,7 @@ __device__ __forceinline__ uint32_t decide_body(const PipeParams& p, DecideSmem<
         uint2* stage = LOCAL ? warpStage : p.staged + static_cast<size_t>(chunk) * chunkSize;
         auto& ring = sm.ring[warp];
         auto& cand = sm.cand[warp];
-        SharedView* shared = &sm.view[SINGLE ? 0u : warp];
+        SharedView* shared = &sm.view[Smem::kViews == 1u ? 0u : warp];
         uint32_t total = 0, kept = 0, total1 = 0;
         uint4* keep = nullptr;
         if constexpr (MODE == kModeFrame1) keep = static_cast<uint4*>(p.keep) + 2u * static_cast<size_t>(chunk) * chunkSize;
@@ -598,15 +602,15 @@ __device__ __forceinline__ uint32_t decide_body(const PipeParams& p, DecideSmem<
         if constexpr (fused_mode(MODE)) stage1 = p.staged2 + static_cast<size_t>(chunk) * chunkSize;
         if constexpr (MODE == kModeRuntime) {
             switch (bv.mode) {
-                case BLZ_MODE_FIRST: total = decide_run_warp<BLZ_MODE_FIRST, SINGLE, OPT>(p.sc, bv, base, limit, stage, ring, cand, surf, shared, flags, keep, kept); break;
-                case BLZ_MODE_LATE: total = decide_run_warp<BLZ_MODE_LATE, SINGLE, OPT>(p.sc, bv, base, limit, stage, ring, cand, surf, shared, flags, keep, kept); break;
-                case BLZ_MODE_TEMPORAL: total = decide_run_warp<BLZ_MODE_TEMPORAL, SINGLE, OPT>(p.sc, bv, base, limit, stage, ring, cand, surf, shared, flags, keep, kept); break;
-                default: total = decide_run_warp<BLZ_MODE_FRUSTUM, SINGLE, OPT>(p.sc, bv, base, limit, stage, ring, cand, surf, shared, flags, keep, kept); break;
+                case BLZ_MODE_FIRST: total = decide_run_warp<BLZ_MODE_FIRST, SINGLE, OPT, Smem::REJECT>(p.sc, bv, base, limit, stage, ring, cand, surf, shared, flags, keep, kept); break;
+                case BLZ_MODE_LATE: total = decide_run_warp<BLZ_MODE_LATE, SINGLE, OPT, Smem::REJECT>(p.sc, bv, base, limit, stage, ring, cand, surf, shared, flags, keep, kept); break;
+                case BLZ_MODE_TEMPORAL: total = decide_run_warp<BLZ_MODE_TEMPORAL, SINGLE, OPT, Smem::REJECT>(p.sc, bv, base, limit, stage, ring, cand, surf, shared, flags, keep, kept); break;
+                default: total = decide_run_warp<BLZ_MODE_FRUSTUM, SINGLE, OPT, Smem::REJECT>(p.sc, bv, base, limit, stage, ring, cand, surf, shared, flags, keep, kept); break;
             }
         } else {
             uint32_t* hist = nullptr;
             if constexpr (MODE == kModeInstanced) hist = p.instHist + static_cast<size_t>(chunk / kInstGroup) * p.instLods;
-            total = decide_run_warp<(MODE < 0 ? 0 : MODE), SINGLE, OPT>(p.sc, bv, base, limit, stage, ring, cand, surf, shared, flags, keep, kept,
+            total = decide_run_warp<(MODE < 0 ? 0 : MODE), SINGLE, OPT, Smem::REJECT>(p.sc, bv, base, limit, stage, ring, cand, surf, shared, flags, keep, kept,
                                                                        stage1, &total1, ready, spinLimit, hist);
         }
         if (!LOCAL && lane == 0) {
