@@ -70,10 +70,12 @@ constexpr uint32_t kInstGroup = 32;
 // frame of 4M objects took 52.3 us without and 48.8 with it, a batch of 64 views 300 and 287. The other
 // single-view passes test every object exactly where it is loaded: most of their lists are short or, in
 // pass 1, mostly inside the frustum, and the second stage's latency cost 0.2 to 0.9 us of passes of 100k to
-// 1M objects (at 4M the instanced pass gained 0.2 us). The kernel that reads each view's pass holds the code of all four, which the bound makes longer: with it 32 views of 500,000 objects, 8 of each pass, took 185 us at
+// 1M objects (at 4M the instanced pass gained 0.2 us). So does the frame in blocks of 128 threads with four objects
+// each (5,000 to 200,000 objects: 8.6 to 11.3 us without, 9.8 to 12.5 with it). The kernel that reads each view's pass holds the
+// code of all four, which the bound makes longer: with it 32 views of 500,000 objects, 8 of each pass, took 185 us at
 // two objects a thread and 307 at four against 169 and 256 without; with one object a thread it is 160 against 221.
-__host__ __device__ constexpr bool reject_mode(int mode, bool single, int opt) {
-    return single ? mode == 5 || mode == 6 : mode != kModeRuntime || opt == 1;
+__host__ __device__ constexpr bool reject_mode(int mode, bool single, int threads, int opt) {
+    return single ? (mode == 5 || mode == 6) && !(threads == 128 && opt == 4) : mode != kModeRuntime || opt == 1;
 }
 static_assert(kModeFrameFused == 5 && kModeFramePyr == 6, "reject_mode names the fused modes");
 
@@ -519,8 +521,8 @@ template <int MODE, bool SINGLE, int THREADS, int OPT>
 struct DecideSmem {
     static constexpr int NW = THREADS / 32;
     using Cand = Candidates<candidate_slots(MODE, SINGLE, OPT)>;
-    using Queue = Ring<reject_mode(MODE, SINGLE, OPT)>;
-    static constexpr bool REJECT = reject_mode(MODE, SINGLE, OPT);
+    using Queue = Ring<reject_mode(MODE, SINGLE, THREADS, OPT)>;
+    static constexpr bool REJECT = reject_mode(MODE, SINGLE, THREADS, OPT);
     static constexpr uint32_t kViews = SINGLE || !REJECT ? 1u : NW;
     static constexpr size_t kUsed = (sizeof(Queue) + sizeof(Cand)) * NW + kViews * sizeof(SharedView);
     static constexpr uint32_t kLods = REJECT && kUsed + 2048 + 1024 <= 48 * 1024 ? 512u : 1u;  // LOD errors
