@@ -1278,17 +1278,13 @@ cudaError_t launch_frame_scatter2(const PipeParams& p1, const PipeParams& p2, cu
     return launch_pdl(cull_scatter2_kernel, g1 + g2, kScatterWarps * 32, 0, s, q1, q2, g1);
 }
 
-// Pass 1's blocks hold a candidate queue beside the survivor ring, which 16 warps do not fit in 48 KB
-// of static shared memory: the 512 x 1 shape runs as twice the blocks of 256 x 1.
-__host__ constexpr uint32_t first_threads(uint32_t threads) { return threads == 512u ? 256u : threads; }
-
 template <int MODE>
 static uint32_t single_blocks_per_sm(uint32_t threads, uint32_t opt) {
     if (threads == 256 && opt == 1) return occupancy_t<MODE, true, 256, 1>();
     if (threads == 256 && opt == 4) return occupancy_t<MODE, true, 256, 4>();
     if (threads == 128 && opt == 2) return occupancy_t<MODE, true, 128, 2>();
     if (threads == 128 && opt == 4) return occupancy_t<MODE, true, 128, 4>();
-    if (threads == 512 && opt == 1) return occupancy_t<MODE, true, MODE == BLZ_MODE_FIRST ? first_threads(512) : 512, 1>();
+    if (threads == 512 && opt == 1) return occupancy_t<MODE, true, 512, 1>();
     return occupancy_t<MODE, true, kObjThreads, kObjOpt>();
 }
 
@@ -1307,7 +1303,6 @@ uint32_t single_chunk_size(uint32_t mode, uint32_t threads, uint32_t opt, uint32
         case kModeInstanced: per = single_blocks_per_sm<kModeInstanced>(threads, opt); break;
         default: per = single_blocks_per_sm<BLZ_MODE_FRUSTUM>(threads, opt); break;
     }
-    if (mode == BLZ_MODE_FIRST) threads = first_threads(threads);
     const uint64_t warps = static_cast<uint64_t>(per) * static_cast<uint64_t>(smCount > 0 ? smCount : 1) * (threads / 32u);
     const uint32_t step = 32u * opt;
     uint64_t size = (count + warps - 1) / warps;
@@ -1352,7 +1347,7 @@ static cudaError_t launch_single_mode(const PipeParams& p, uint32_t threads, uin
     if (threads == 256 && opt == 4) return launch_t<MODE, true, 256, 4>(p, 0, smCount, s);
     if (threads == 128 && opt == 2) return launch_t<MODE, true, 128, 2>(p, 0, smCount, s);
     if (threads == 128 && opt == 4) return launch_t<MODE, true, 128, 4>(p, 0, smCount, s);
-    if (threads == 512 && opt == 1) return launch_t<MODE, true, MODE == BLZ_MODE_FIRST ? first_threads(512) : 512, 1>(p, 0, smCount, s);
+    if (threads == 512 && opt == 1) return launch_t<MODE, true, 512, 1>(p, 0, smCount, s);
     return launch_t<MODE, true, kObjThreads, kObjOpt>(p, 0, smCount, s);
 }
 
