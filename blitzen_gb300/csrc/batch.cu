@@ -349,18 +349,23 @@ int blz_autotune_batch(blz_ctx* c, const BlzBatchView* views, uint32_t n, uint32
     if (!c || !views || n == 0) return fail(BLZ_ERR_INVALID_ARGUMENT, "ctx or views is NULL");
     if (c->capturing) return fail(BLZ_ERR_INVALID_ARGUMENT, "the autotuner cannot run inside a capture");
     const uint64_t objects = batch_objects(c, views, n);
-    if (const TunedShape* t = find_tuned(c, objects, n, kTunedBatch)) {
-        c->shape = t->shape;
-        if (best) *best = t->shape;
-        if (bestUs) *bestUs = t->us;
+    auto keep = [&](const TunedShape& t) {
+        c->shape = t.shape;
+        if (best) {
+            *best = t.shape;
+            best->chunkObjects = batch_chunk(t.shape);
+        }
+        if (bestUs) *bestUs = t.us;
         return BLZ_OK;
-    }
+    };
+    if (const TunedShape* t = find_tuned(c, objects, n, kTunedBatch)) return keep(*t);
     if (repeats == 0) repeats = 5;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const uint32_t threads[] = {128, 256, 512};
     const uint32_t opts[] = {1, 2, 4, 8};
     const uint32_t perSm[] = {0, 1, 2, 4};
-    const uint32_t chunks[] = {256, 512, 1024};
+    const uint32_t chunks[] = {0, 256, 512, 1024};
+    const bool uniform = uniform_mode(views, n) >= 0;
     cudaEvent_t a, b;
     cudaEventCreate(&a);
     cudaEventCreate(&b);
@@ -373,6 +378,15 @@ int blz_autotune_batch(blz_ctx* c, const BlzBatchView* views, uint32_t n, uint32
                     if (s && s * t > 2048) continue;
                     if (!batch_shape_supported(t, o)) continue;
                     const BlzLaunchShape sh{t, o, s, k};
+                    // The default shape's own chunk (0) is cut for small batches and a candidate beside the named
+                    // ones; in the other shapes it is 512. Candidates that run the same kernel over the same chunks
+                    // as another are left out: 256 x 2 over a named chunk where all views run one pass (256 x 1), and
+                    // 512 where that is the default's own.
+                    const bool byDefault = t == kObjThreads && o == kObjOpt;
+                    if (k == 0 && !byDefault) continue;
+                    if (k != 0 && byDefault && uniform) continue;
+                    const BlzLaunchShape own{kObjThreads, kObjOpt, s, 0};
+                    if (k != 0 && (byDefault || (uniform && t == kObjThreads && o == 1)) && batch_chunk_for(own, objects, c->smCount) == k) continue;
                     if (run_batch_shape(c, views, n, objects, st, sh) != BLZ_OK) continue;  // warm-up
                     cudaEventRecord(a, st);
                     int rc = BLZ_OK;
@@ -391,11 +405,9 @@ int blz_autotune_batch(blz_ctx* c, const BlzBatchView* views, uint32_t n, uint32
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     if (!(topUs < 1e30f)) return fail(BLZ_ERR_CUDA, "no launch shape ran");
-    c->shape = top;
-    remember_tuned(c, TunedShape{objects, n, kTunedBatch, top, topUs});
-    if (best) *best = top;
-    if (bestUs) *bestUs = topUs;
-    return BLZ_OK;
+    const TunedShape tuned{objects, n, kTunedBatch, top, topUs};
+    remember_tuned(c, tuned);
+    return keep(tuned);
 }
 
 int blz_batch_graph_create(blz_ctx* c, const BlzBatchView* views, uint32_t n, blz_stream_t stream, blz_batch_graph** outGraph) {

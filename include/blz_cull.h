@@ -405,8 +405,10 @@ int blz_batch_graph_destroy(blz_batch_graph* g);
  * blz_autotune_batch times every batch shape (threads x objects per thread x blocks per SM x chunk
  * size) on the given batch, keeps the fastest as the context's shape and caches it for the batch's
  * size (total objects, view count): later batches of that size use it, whatever the context's
- * shape, and a later call for that size returns the cached choice without timing again. The
- * reference has one fixed shape, N/64 + 1 groups of 64 threads (blitML.h:64-67). */
+ * shape, and a later call for that size returns the cached choice without timing again. The default
+ * shape's own chunk (0) is among the candidates; where it is the fastest, the context's shape has the
+ * chunk 0 and best names 512. The reference has one fixed shape, N/64 + 1 groups of 64 threads
+ * (blitML.h:64-67). */
 typedef struct BlzLaunchShape {
     uint32_t threadsPerBlock;
     uint32_t objectsPerThread;
