@@ -416,14 +416,7 @@ __device__ __forceinline__ void load_transform(const SceneTables& sc, uint32_t t
 // written (any table, list, depth buffer, count) is read after that with plain loads, never with the
 // read-only (.nc) ones, which promise the memory constant from the kernel's start and which the
 // compiler may move above the wait.
-#ifndef BLZ_TRIG
-#define BLZ_TRIG 0
-#endif
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory");
-#if BLZ_TRIG
- asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-#endif
-}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ void st_release_gpu(unsigned int* p, unsigned int v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
