@@ -1713,4 +1713,36 @@ cudaError_t launch_batch_cull(const PipeParams& p, uint32_t threads, uint32_t op
     return cudaErrorInvalidValue;
 }
 
+// Asking for a kernel's attributes loads it.
+template <typename K>
+static cudaError_t load_kernel(K* kernel) {
+    cudaFuncAttributes a;
+    return cudaFuncGetAttributes(&a, reinterpret_cast<const void*>(kernel));
+}
+
+cudaError_t load_batch_kernels(uint32_t threads, uint32_t opt) {
+    cudaError_t e = cudaSuccess;
+    auto load = [&](auto* kernel) {
+        if (e == cudaSuccess) e = load_kernel(kernel);
+    };
+    load(batch_order_kernel);
+    load(batch_scan_kernel);
+    load(batch_scan_warp_kernel);
+    load(batch_scatter_kernel);
+    if (threads == 256 && opt <= 2) {
+        load(cull_decide_kernel<BLZ_MODE_FRUSTUM, false, 256, 1>);
+        load(cull_decide_kernel<BLZ_MODE_TEMPORAL, false, 256, 1>);
+    } else if (threads == 512 && opt == 1) {
+        load(cull_decide_kernel<BLZ_MODE_FRUSTUM, false, 512, 1>);
+        load(cull_decide_kernel<BLZ_MODE_TEMPORAL, false, 512, 1>);
+    }
+#define BLZ_BATCH_CASE(T, O) \
+    if (threads == T && opt == O) load(cull_decide_kernel<kModeRuntime, false, T, O>);
+    BLZ_BATCH_CASE(128, 1) BLZ_BATCH_CASE(128, 2) BLZ_BATCH_CASE(128, 4) BLZ_BATCH_CASE(128, 8)
+    BLZ_BATCH_CASE(256, 1) BLZ_BATCH_CASE(256, 2) BLZ_BATCH_CASE(256, 4)
+    BLZ_BATCH_CASE(512, 1) BLZ_BATCH_CASE(512, 2)
+#undef BLZ_BATCH_CASE
+    return e;
+}
+
 }  // namespace blz

@@ -263,6 +263,9 @@ bool batch_shape_supported(uint32_t threads, uint32_t opt);
 // mode: the pass every view of the batch runs, or -1 when they differ (the kernel reads it per view)
 cudaError_t launch_batch_cull(const PipeParams& p, uint32_t threads, uint32_t opt, uint32_t blocksPerSm, int smCount,
                               cudaStream_t s, int mode);
+// Loads the kernels of frustum and temporal batches of a shape on the current device (a kernel is otherwise loaded by
+// its first launch, milliseconds each).
+cudaError_t load_batch_kernels(uint32_t threads, uint32_t opt);
 uint32_t instanced_tile_size();
 // Above this many LODs the instanced cull's scratch is a block of its own, and a recorded call runs as one
 // launch without scratch (launch_instanced_cull).
@@ -287,6 +290,7 @@ cudaError_t launch_transforms_rotate(const BlzMeshTransform* table, uint32_t tab
                                      uint32_t dynCount, const uint32_t* ids, const float* axes, float angle, uint32_t n,
                                      BlzMeshTransform* dst, unsigned int* status, cudaStream_t s);
 // *word += n on the stream (one thread).
+cudaError_t load_transform_kernels();
 cudaError_t launch_add_word(unsigned int* word, unsigned int n, cudaStream_t s);
 // *out = atomicExch(status, 0) on the stream (one thread).
 cudaError_t launch_take_status(unsigned int* status, unsigned int* out, cudaStream_t s);

@@ -68,6 +68,11 @@ cudaError_t launch_transforms_rotate(const BlzMeshTransform* table, uint32_t tab
                       cs, n, dst, status);
 }
 
+cudaError_t load_transform_kernels() {
+    cudaFuncAttributes a;
+    return cudaFuncGetAttributes(&a, reinterpret_cast<const void*>(transforms_rotate_kernel));
+}
+
 // ------------------------------------------------------------------ occluder raster
 
 struct BoxRect {

@@ -27,6 +27,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/blz_cull.h"
+#include "kernels.h"
 
 namespace {
 
@@ -313,6 +314,12 @@ int blz_serve_create(blz_ctx* ctx, const BlzServeConfig* config, blz_server** ou
             return rc;
         }
     }
+    // the kernels of its batches are loaded here and not while a first request waits (21 ms, once a process)
+    BlzLaunchShape shape;
+    blz_get_launch_shape(ctx, &shape);
+    (void)blz::load_transform_kernels();
+    (void)blz::load_batch_kernels(shape.threadsPerBlock, shape.objectsPerThread);
+    (void)cudaGetLastError();
     blz_server* raw = s.release();
     raw->worker = std::thread([raw] { raw->run(); });
     *out = raw;
