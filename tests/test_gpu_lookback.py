@@ -1,13 +1,14 @@
 """The bounded look-back of the instanced cull of many LODs, in the recorded form that waits: its waits run
 out when its ticket has been advanced, and the replay after that equals the oracle. A direct call after the
-hook takes that form as well (one launch), the one after it the counting sort again (four)."""
+hook takes that form as well (one launch), the one after it the counting sort again (four); so does a call of a
+few objects, which are one tile and wait for none."""
 import numpy as np
 import pytest
 import torch
 
 from blitzen_gb300 import abi
 from blitzen_gb300 import scenes as S
-from blitzen_gb300.culler import Culler, Target
+from blitzen_gb300.culler import Culler, Target, to_device
 from oracle import oracle as O
 from tests.helpers import assert_records_equal, view_for
 
@@ -61,6 +62,22 @@ def test_recorded_lookback_runs_out_then_recovers(lib, advance):
             graphs[1].launch()
             assert c.check() == 0
         p.check()
+
+
+@pytest.mark.parametrize("n,launches", [(1, 1), (32, 1), (128, 1), (129, 4), (5000, 4)])
+def test_few_objects_take_one_launch(lib, n, launches):
+    with Culler(0) as c:
+        p = Pass(c)
+        objs = np.ascontiguousarray(p.sc.objects[:n])
+        d = to_device(objs, "cuda")
+        before = c.launches
+        c.draw_instance_cull_pass(p.v, p.dctr, p.inst, SLOTS, p.t, objects=d, count=n)
+        assert c.launches - before == launches
+        assert c.check() == 0
+        cnt, cmds, octr, oinst, _ = O.cull_instanced(p.v, p.sc, p.ctr, p.cap, SLOTS, objects=objs)
+        assert_records_equal(p.t.read(), (cnt, cmds), "commands")
+        assert np.array_equal(p.dctr.cpu().numpy().view(np.uint32), octr.view(np.uint32).reshape(-1))
+        assert np.array_equal(p.inst.cpu().numpy().view(np.uint32), oinst)
 
 
 def test_direct_call_after_the_hook_takes_the_waiting_form(lib):
