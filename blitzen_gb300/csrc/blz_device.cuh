@@ -403,10 +403,14 @@ __device__ __forceinline__ void ldg_transform(const BlzMeshTransform* t, float4&
 
 // Transform `tid` of the scene, from the bound dynamic rows when tid < dynCount (device or pinned
 // host memory), else from the resident table: a pointer select, then one 32-byte load (both are
-// 32-byte aligned).
+// 32-byte aligned). An ordinary load, which the kernels that have no ring to fill want in flight together with others.
 __device__ __forceinline__ void load_transform(const SceneTables& sc, uint32_t tid, float4& posScale, float4& q) {
     const BlzMeshTransform* base = tid < sc.dynCount ? sc.dynRows : sc.transforms;
-    ldg_transform(base + tid, posScale, q);
+    const double4_32a x = *reinterpret_cast<const double4_32a*>(base + tid);
+    auto lo = [](double d) { return __int_as_float(__double2loint(d)); };
+    auto hi = [](double d) { return __int_as_float(__double2hiint(d)); };
+    posScale = make_float4(lo(x.x), hi(x.x), lo(x.y), hi(x.y));
+    q = make_float4(lo(x.z), hi(x.z), lo(x.w), hi(x.w));
 }
 
 // Programmatic dependent launch. A kernel launched with programmatic stream serialization

@@ -19,6 +19,7 @@ constexpr int kInstOpt = 8;
 constexpr int kInstWarps = kInstThreads / 32;
 constexpr uint32_t kInstTile = kInstThreads * kInstOpt;
 constexpr uint32_t kNoBucket = 0xFFFFFFFFu;
+constexpr uint32_t kInstCmdBatch = 4;  // LODs whose offsets and records' fields are loaded together
 
 // Frustum + LOD decision (drawInstCull.cs.hlsl:22-36). Returns the global LOD id or kNoBucket.
 __device__ __forceinline__ uint32_t inst_bucket(const SceneTables& sc, const BlzRenderObject* objects, uint32_t i,
@@ -95,6 +96,9 @@ __global__ void __launch_bounds__(kInstThreads) cull_instanced_kernel(const Inst
         const uint32_t i = wbase + k * 32u + lane;
         bucket[k] = (i < p.count) ? inst_bucket(p.sc, p.objects, i, v, flags) : kNoBucket;
     }
+    uint32_t listAt[kInstOpt];  // on its way while the tile waits; a load cannot pass the stores
+#pragma unroll
+    for (int k = 0; k < kInstOpt; ++k) listAt[k] = bucket[k] != kNoBucket ? ldp(&p.counters[bucket[k]].instanceOffset) : 0u;
 #pragma unroll
     for (int k = 0; k < kInstOpt; ++k) {
         const unsigned peers = __match_any_sync(0xFFFFFFFFu, bucket[k]);
@@ -155,7 +159,7 @@ __global__ void __launch_bounds__(kInstThreads) cull_instanced_kernel(const Inst
         if (bucket[k] == kNoBucket) continue;
         const uint32_t b = bucket[k];
         const uint32_t pos = bucketBase[b] + hist[warp * nL + b] + off[k];
-        const uint64_t at = static_cast<uint64_t>(ldp(&p.counters[b].instanceOffset)) + pos;
+        const uint64_t at = static_cast<uint64_t>(listAt[k]) + pos;
         if (pos < slots && at < p.instanceCapacity) p.instances[at] = wbase + k * 32u + lane;
         else flags |= BLZ_FLAG_INSTANCE_OVERFLOW;
     }
@@ -191,24 +195,35 @@ __global__ void __launch_bounds__(kInstThreads) cull_instanced_kernel(const Inst
         }
         running = warpOff + incl - mine;
         unsigned int f = 0u;
-        for (uint32_t b = b0; b < b1; ++b) {
-            const uint32_t total = hist[b];
-            p.counters[b].instanceCount = total;
-            if (total > slots || static_cast<uint64_t>(ldp(&p.counters[b].instanceOffset)) + min(total, slots) > p.instanceCapacity)
-                f |= BLZ_FLAG_INSTANCE_OVERFLOW;
-            if (total == 0u) continue;
-            if (running < p.capacity) {
-                uint8_t* rec = p.cmds + static_cast<size_t>(running) * p.stride;
-                uint32_t* w = reinterpret_cast<uint32_t*>(rec);
-                const uint2 lod = ldp(reinterpret_cast<const uint2*>(p.sc.lods + b));
-                w[0] = ldp(&p.counters[b].instanceOffset);
-                w[1] = lod.x;
-                w[2] = min(total, slots);
-                w[3] = lod.y;
-                w[4] = 0u;
-                w[5] = 0u;
+        for (uint32_t first = b0; first < b1; first += kInstCmdBatch) {
+            uint32_t offset[kInstCmdBatch];  // a batch's loads together, before its stores
+            uint2 lod[kInstCmdBatch];
+#pragma unroll
+            for (uint32_t k = 0; k < kInstCmdBatch; ++k) {
+                const uint32_t b = min(first + k, nL - 1u);
+                offset[k] = ldp(&p.counters[b].instanceOffset);
+                lod[k] = ldp(reinterpret_cast<const uint2*>(p.sc.lods + b));
             }
-            ++running;
+#pragma unroll
+            for (uint32_t k = 0; k < kInstCmdBatch; ++k) {
+                const uint32_t b = first + k;
+                if (b >= b1) break;
+                const uint32_t total = hist[b];
+                p.counters[b].instanceCount = total;
+                if (total > slots || static_cast<uint64_t>(offset[k]) + min(total, slots) > p.instanceCapacity)
+                    f |= BLZ_FLAG_INSTANCE_OVERFLOW;
+                if (total == 0u) continue;
+                if (running < p.capacity) {
+                    uint32_t* w = reinterpret_cast<uint32_t*>(p.cmds + static_cast<size_t>(running) * p.stride);
+                    w[0] = offset[k];
+                    w[1] = lod[k].x;
+                    w[2] = min(total, slots);
+                    w[3] = lod[k].y;
+                    w[4] = 0u;
+                    w[5] = 0u;
+                }
+                ++running;
+            }
         }
         if (all > p.capacity) f |= BLZ_FLAG_COMMAND_OVERFLOW;
         if (f) atomicOr(&s_flags, f);
