@@ -16,7 +16,6 @@ constexpr size_t kDefaultStateCapacity = size_t(1) << 22;  // 4M tile states (32
 constexpr size_t kPinnedBytes = size_t(8) << 20;            // pinned host staging: transform rows, batch views
 constexpr size_t kFirstManyLodsBytes = size_t(4) << 20;     // many-LOD instanced scratch of a new context
 constexpr uint32_t kInstSortedMinObjects = 128;             // lists of many LODs up to here: the one-launch form
-constexpr uint32_t kMaxInstancedLods = 4096;                // shared-memory bucket histograms
 
 // An autotuner's choice for one workload size: batches keyed by (total objects, views), single-view
 // passes by (objects, 1, pass).

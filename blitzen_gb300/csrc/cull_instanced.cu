@@ -252,8 +252,10 @@ cudaError_t launch_instanced_cull(const InstancedParams& p, const BlzCameraViewD
     if (tiles == 0) tiles = 1;
     const size_t smem = instanced_smem_bytes(p.sc.lodCount);
     if (smem > 48 * 1024) {
+        // the limit is the process's, so it is never this call's own size: another thread's launch, or a graph about to be
+        // instantiated, may need more
         cudaError_t e = cudaFuncSetAttribute(cull_instanced_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(smem));
+                                             static_cast<int>(instanced_smem_bytes(kMaxInstancedLods)));
         if (e != cudaSuccess) return e;
     }
     return launch_pdl(cull_instanced_kernel, tiles, kInstThreads, smem, s, p, view);

@@ -1668,7 +1668,8 @@ cudaError_t launch_instanced_staged(const PipeParams& p, const InstStagedParams&
     const uint32_t warps = inst_warps(q.nL), threads32 = warps * 32u;
     const size_t rowBytes = sizeof(uint32_t) * (warps + 2u + inst_parts(q.nL, threads32)) * inst_stride(q.nL);
     if (rowBytes > 48 * 1024) {
-        e = cudaFuncSetAttribute(inst_place_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(rowBytes));
+        // the limit is the process's, so it is never this call's own size: another thread's launch may be under way with more
+        e = cudaFuncSetAttribute(inst_place_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kInstSmem));
         if (e != cudaSuccess) return e;
     }
     return launch_pdl(inst_place_kernel, q.groups, threads32, rowBytes, s, q);

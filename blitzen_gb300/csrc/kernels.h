@@ -266,6 +266,7 @@ cudaError_t launch_batch_cull(const PipeParams& p, uint32_t threads, uint32_t op
 // Loads the kernels of frustum and temporal batches of a shape on the current device (a kernel is otherwise loaded by
 // its first launch, milliseconds each).
 cudaError_t load_batch_kernels(uint32_t threads, uint32_t opt);
+constexpr uint32_t kMaxInstancedLods = 4096;  // shared-memory bucket histograms
 uint32_t instanced_tile_size();
 // Above this many LODs the instanced cull's scratch is a block of its own, and a recorded call runs as one
 // launch without scratch (launch_instanced_cull).
