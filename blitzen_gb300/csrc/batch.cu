@@ -3,9 +3,10 @@
 //
 // The reference culls one camera per pass with one dispatch each (src/Core/blitzenEngine.h:49,
 // src/Renderer/BlitzenVulkan/vulkanDraw.cpp:107-226). Here every (view, chunk) pair is an item of
-// one decide launch (chunks of 256, 512 or 1024 objects, the launch shape's chunk size): warps start on the chunk of their index and take further chunks
-// from a work counter, and the scatter launch turns the per-chunk counts into per-view offsets and
-// draw counts, so views of 1k and 2M objects share the machine without a launch or a tail per view.
+// one decide launch (chunks of the launch shape's 256, 512 or 1024 objects, or down to 64 where a small batch
+// is cut finer, batch_chunk_for): warps start on the chunk of their index and take further chunks from a work
+// counter. A scan launch turns the per-chunk counts into per-view offsets and draw counts, and a scatter launch
+// writes the records, so views of 1k and 2M objects share the machine without a launch or a tail per view.
 #include <algorithm>
 #include <cstddef>
 #include <cstring>

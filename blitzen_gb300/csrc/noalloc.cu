@@ -5,7 +5,7 @@
 // memory that grows on demand, and growing it means cudaFree + cudaMalloc. Some callers cannot take that: a frame loop that has reserved all of its
 // device memory up front (another pool owns the rest, so a cudaMalloc would fail mid-frame), or
 // one that must never stall, since cudaFree waits for the whole device. This entry point runs the
-// same two kernels with that staging in `g_noallocScratch` below, a file-scope array sized for at
+// same kernels (two, or one for a short list) with that staging in `g_noallocScratch` below, a file-scope array sized for at
 // most BLZ_NOALLOC_MAX_OBJECTS render objects, and rejects larger lists instead of growing.
 //
 // Set-up: the array's device address is fetched with cudaGetSymbolAddress by the first call made on
